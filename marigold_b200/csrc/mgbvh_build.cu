@@ -1675,7 +1675,7 @@ struct MNodeExtra {
 // Shared memory of one subtree CTA for subtrees of up to kCap objects: the
 // records, two index lists, two node lists (every listed node holds more than
 // 32 objects and the nodes of one list are disjoint, so kCap / 33 + 1 entries
-// suffice), per-warp bins and exchange space.
+// suffice) and per-warp bins.
 template <uint32_t kCap>
 struct MediumSmemT {
     static constexpr uint32_t kListCap = kCap / (kSmallMax + 1) + 1;
@@ -1685,7 +1685,6 @@ struct MediumSmemT {
     MNode list[2][kListCap];
     MNodeExtra list_x[2][kListCap];
     uint32_t bins[kMediumWarps][kBinWords];
-    XRec xchg[kMediumWarps][32];
     uint32_t list_n[2];
     uint32_t rootk[12];
 };
@@ -1706,9 +1705,11 @@ struct SmallRef {
 
 // The persistent build's subtree CTA: the records, lists and bins of a
 // subtree CTA, plus the list of its subtrees of <= 32 objects (at most
-// kCap / 2: disjoint subtrees of at least 2 objects).
+// kCap / 2: disjoint subtrees of at least 2 objects) and each warp's tables
+// to build them.
 template <uint32_t kCap>
 struct MediumSmemQ : MediumSmemT<kCap> {
+    SubtreeSmem tables[kMediumWarps];
     SmallRef sref[kCap / 2];
     uint32_t sref_n;
 };
@@ -1993,7 +1994,7 @@ __global__ void transpose_weights_kernel(const __nv_bfloat16* __restrict__ w, __
 // kQueue (the persistent batched build): records are read through L2 only,
 // and each subtree of <= 32 objects is built at once by the warp that split
 // it off, from shared memory, instead of going to the small list.
-template <bool kLearn, class MS, bool kQueue = false, bool kSmallLevels = true>
+template <bool kLearn, class MS, bool kQueue = false, bool kGeneral = false>
 __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec* rec1,
                                             Task* small, uint32_t cap_small, const Params& P,
                                             const Out& O, const Learn& LN) {
@@ -2328,12 +2329,8 @@ __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec*
                 shi[1] = b.y;
                 shi[2] = b.z;
             }
-            if constexpr (kSmallLevels)
-                warp_build_subtree_levels(slo, shi, sid, q.len, base + q.cs, q.slot, q.pair, q.depth, t.nbase,
-                                          t.tbase, q.b, P, O, S.xchg[warp]);
-            else
-                warp_build_subtree(slo, shi, sid, q.len, base + q.cs, q.slot, q.pair, q.depth, t.nbase, t.tbase, q.b,
-                                   P, O, S.xchg[warp]);
+            warp_build_subtree<kGeneral>(slo, shi, sid, q.len, base + q.cs, q.slot, q.pair, q.depth, t.nbase, t.tbase, q.b, P, O,
+                               S.tables[warp]);
         }
     }
 }
@@ -2486,24 +2483,20 @@ __global__ void __launch_bounds__(256) small_select_kernel(const Task* __restric
 
 // ---------------------------------------------------------------- small
 
-// One warp per subtree of <= 32 objects. kLevels: the level-synchronous
-// builder (every node adaptive with one threshold per object); otherwise the
-// depth-first builder that also covers binned nodes and fixed step counts.
-// kMinBlocks: CTAs of 256 threads per SM the register budget allows (the
-// context's small-subtree occupancy): 3 (80 registers, 24 warps per SM) or 2
-// (126 registers, 16 warps). The kernel is issue-bound on fixed-latency
-// dependencies; on the noisy icosphere the extra warps hide more of them than
-// the spills of the tighter budget add (warp-subtree phase 0.568 -> 0.543 ms;
-// 4 CTAs at 64 registers: 0.594 ms), while the batched scene builds 3% faster
-// at 16 warps. The autotuner picks it per workload.
-template <bool kLevels, int kMinBlocks>
+// One warp per subtree of <= 32 objects. kGeneral: any split profile;
+// otherwise the reference's own (every node adaptive with one threshold per
+// object). kMinBlocks: CTAs of 256 threads per SM that the register budget
+// must allow (the context's small-subtree occupancy, warps per SM / 8): 3 (80
+// registers, 0.386 ms on the level-8 icosphere) or 2 (112 registers, 0.426 ms);
+// 4 (64 registers) spills more than its warps hide, 0.412 ms.
 // range (nullable): build tasks [range[0], range[1]) instead of all of them.
+template <bool kGeneral, int kMinBlocks>
 __global__ void __launch_bounds__(256, kMinBlocks) small_kernel(const Task* __restrict__ tasks,
                                                    const Rec* __restrict__ rec0,
                                                    const Rec* __restrict__ rec1, Params P, Out O,
                                                    const uint32_t* range) {
     pdl_enter();
-    __shared__ XRec xchg[8][32];
+    __shared__ SubtreeSmem tables[8];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const uint32_t w0 = range ? range[0] : 0u;
     const uint32_t n_tasks = range ? range[1] : *reinterpret_cast<volatile uint32_t*>(&O.ctr->n_small);
@@ -2535,12 +2528,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) small_kernel(const Task* __re
             hi[2] = r.hi.z;
         }
         const float b[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
-        if constexpr (kLevels)
-            warp_build_subtree_levels(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase,
-                                      t.tbase, b, P, O, xchg[wib]);
-        else
-            warp_build_subtree(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase, t.tbase,
-                               b, P, O, xchg[wib]);
+        warp_build_subtree<kGeneral>(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase, t.tbase, b, P, O,
+                           tables[wib]);
     }
 }
 
@@ -2901,16 +2890,16 @@ __device__ __noinline__ void queue_large_task(const QueueArgs& Q, LargeSmem& L, 
 // The persistent build's subtree CTA and warp-subtree tasks, as separate
 // (not inlined) functions: each gets its own register allocation instead of
 // the union of every task kind's.
-template <uint32_t kCap, bool kLevels>
+template <uint32_t kCap, bool kGeneral>
 __device__ __noinline__ void queue_medium_task(MediumSmemQ<kCap>& S, const Task& t, Rec* rec0, Rec* rec1,
                                                const Params& P, const Out& O) {
-    medium_task<false, MediumSmemQ<kCap>, true, kLevels>(S, t, rec0, rec1, nullptr, 0u, P, O,
-                                                         Learn{nullptr, 0, nullptr, 0, nullptr});
+    medium_task<false, MediumSmemQ<kCap>, true, kGeneral>(S, t, rec0, rec1, nullptr, 0u, P, O,
+                                                Learn{nullptr, 0, nullptr, 0, nullptr});
 }
 
-template <bool kLevels>
+template <bool kGeneral>
 __device__ __noinline__ void queue_small_task(const Task& t, const Rec* rec0, const Rec* rec1, const Params& P,
-                                              const Out& O, XRec* xchg) {
+                                              const Out& O, SubtreeSmem& tables) {
     const uint32_t lane = threadIdx.x & 31u;
     const Rec* src = (t.buf ? rec1 : rec0) + t.start;
     float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
@@ -2926,14 +2915,10 @@ __device__ __noinline__ void queue_small_task(const Task& t, const Rec* rec0, co
         hi[2] = r.hi.z;
     }
     const float b[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
-    if constexpr (kLevels)
-        warp_build_subtree_levels(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase, t.tbase, b, P, O,
-                                  xchg);
-    else
-        warp_build_subtree(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase, t.tbase, b, P, O, xchg);
+    warp_build_subtree<kGeneral>(lo, hi, id, t.len, t.start, t.slot, t.pair, t.depth, t.nbase, t.tbase, b, P, O, tables);
 }
 
-template <uint32_t kCap, bool kLevels>
+template <uint32_t kCap, bool kGeneral>
 __global__ void __launch_bounds__(kMediumThreads, MGBVH_QUEUE_MIN_BLOCKS)
     queue_build_kernel(QueueArgs Q, Rec* rec0, Rec* rec1, Params P, Out O) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2951,9 +2936,9 @@ __global__ void __launch_bounds__(kMediumThreads, MGBVH_QUEUE_MIN_BLOCKS)
         if (t.len > P.medium_max)
             queue_large_task(Q, L, t, Q.qcb + 6 * p.idx, rec0, rec1, P, O);
         else if (t.len > kSmallMax)
-            queue_medium_task<kCap, kLevels>(S, t, rec0, rec1, P, O);
+            queue_medium_task<kCap, kGeneral>(S, t, rec0, rec1, P, O);
         else if (warp == 0)  // a subtree of <= 32 objects split off a node above medium_max
-            queue_small_task<kLevels>(t, rec0, rec1, P, O, S.xchg[0]);
+            queue_small_task<kGeneral>(t, rec0, rec1, P, O, S.tables[0]);
         __threadfence();
         __syncthreads();
         if (threadIdx.x == 0) atomicSub(&Q.st->pending, 1u);
@@ -3654,9 +3639,8 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
                     tasks, rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
         };
         // small subtrees: count read on the device; grid sized for full occupancy
-        const bool lv_small = P.adaptive_steps == 0 && P.adaptive_max_n == kSmallMax;
-        auto small = ctx->small_warps == 16u ? (lv_small ? small_kernel<true, 2> : small_kernel<false, 2>)
-                                             : (lv_small ? small_kernel<true, 3> : small_kernel<false, 3>);
+        auto small = ctx->small_warps == 16u ? (subtree_general(P) ? small_kernel<true, 2> : small_kernel<false, 2>)
+                                             : (subtree_general(P) ? small_kernel<true, 3> : small_kernel<false, 3>);
         // as many warps as 8 CTAs of 256 threads per SM, whatever the CTA size
         const int small_grid = ctx->sm_count * (2048 / (int)ctx->small_threads);
         if (ctx->stream_slots && ctx->h_nodes_out) {
@@ -4206,15 +4190,15 @@ int enqueue_batch(mgbvh_ctx* ctx, const BatchPlan& B, const Caps& C, const mgbvh
         MG_CUDA(cudaGetLastError());
         if (!fixed_levels) MG_CUDA(cudaEventRecord(ctx->evp[0], sm));
         const bool small_cap = P.medium_max <= kMediumSmallCap;
-        const bool lv = P.adaptive_steps == 0 && P.adaptive_max_n == kSmallMax;
+        const bool gen = subtree_general(P);
         const size_t smem = small_cap ? sizeof(MediumSmemQ<kMediumSmallCap>) : sizeof(MediumSmemQ<kMediumMax>);
         int grid = small_cap ? ctx->queue_ctas[0] : ctx->queue_ctas[1];
         if (ctx->queue_per_sm) grid = std::min(grid, ctx->sm_count * (int)ctx->queue_per_sm);
-        if (small_cap && lv)
+        if (small_cap && gen)
             queue_build_kernel<kMediumSmallCap, true><<<grid, kMediumThreads, smem, sm>>>(Q, rec0, rec1, P, O);
         else if (small_cap)
             queue_build_kernel<kMediumSmallCap, false><<<grid, kMediumThreads, smem, sm>>>(Q, rec0, rec1, P, O);
-        else if (lv)
+        else if (gen)
             queue_build_kernel<kMediumMax, true><<<grid, kMediumThreads, smem, sm>>>(Q, rec0, rec1, P, O);
         else
             queue_build_kernel<kMediumMax, false><<<grid, kMediumThreads, smem, sm>>>(Q, rec0, rec1, P, O);
@@ -5097,7 +5081,7 @@ int mgbvh_build_aabbs_noalloc(const float* d_aabbs, uint32_t count, const mgbvh_
             nullptr);
     if (cls != 0) {
         const int grid = std::max(1, std::min(sms, (int)((n / 2 + 8 + 7) / 8)));
-        if (P.adaptive_steps == 0 && P.adaptive_max_n == kSmallMax)
+        if (subtree_general(P))
             small_kernel<true, 3><<<grid, 256, 0, sm>>>(S->small, S->rec, S->rec, P, O, nullptr);
         else
             small_kernel<false, 3><<<grid, 256, 0, sm>>>(S->small, S->rec, S->rec, P, O, nullptr);

@@ -1,11 +1,8 @@
 // mgbvh_device.cuh — device-side types and the warp subtree builder.
 //
-// A subtree whose root holds at most 32 objects is built by one warp with
-// the objects in registers: lane i holds the object at position i of the
-// subtree's range. The warp visits the subtree's nodes depth first; for each
-// node it evaluates every candidate split of the reference's select_split
-// (bvh/src/lib.rs:493-534) in parallel, one candidate per lane, and applies
-// the winner with a stable ballot partition of the lanes.
+// A subtree whose root holds at most 32 objects is built by one warp, all nodes
+// of one depth at a time (warp_build_subtree below): each node is a range of
+// lanes, and object sets are 32-bit masks over the subtree's sorted orders.
 #pragma once
 
 #include <cstdint>
@@ -180,15 +177,6 @@ __device__ __forceinline__ void box_grow2(float* a, float* b, bool first, float 
     }
 }
 
-// Warp union of the boxes of the lanes in `mask` (exact: min/max on keys).
-__device__ __forceinline__ void warp_box_union(bool in, const float* lo, const float* hi,
-                                               float* out) {
-    for (int a = 0; a < 3; ++a) {
-        out[a] = funkey(__reduce_min_sync(kFull, in ? fkey(lo[a]) : kKeyPosInf));
-        out[3 + a] = funkey(__reduce_max_sync(kFull, in ? fkey(hi[a]) : kKeyNegInf));
-    }
-}
-
 // 64-bit candidate key: total_cmp(cost), then axis, then candidate index —
 // the first minimum of min_by over axes of min_by over candidates.
 __device__ __forceinline__ uint64_t cand_key(float cost, uint32_t axis, uint32_t idx) {
@@ -324,315 +312,21 @@ __device__ __forceinline__ void shfl_cand(Cand& c, uint32_t src) {
     }
 }
 
-struct XRec {
-    float4 lo;  // min xyz, object id (bits)
-    float4 hi;  // max xyz, unused
-};
-
-// Stable partition of the lanes of segment [s, s+n): lanes with `pred` move
-// to the front in lane order, the others follow in lane order. The records
-// travel through the warp's exchange area.
-__device__ __forceinline__ void warp_stable_permute(bool in_seg, bool pred, uint32_t s, uint32_t n_lt,
-                                                    uint32_t lane, float* lo, float* hi,
-                                                    uint32_t& id, XRec* x) {
-    const uint32_t ltm = __ballot_sync(kFull, in_seg && pred);
-    const uint32_t segm = __ballot_sync(kFull, in_seg);
-    const uint32_t below = (1u << lane) - 1u;
-    const uint32_t dst = pred ? s + __popc(ltm & below) : s + n_lt + __popc(segm & ~ltm & below);
-    if (in_seg) {
-        x[dst].lo = make_float4(lo[0], lo[1], lo[2], __uint_as_float(id));
-        x[dst].hi = make_float4(hi[0], hi[1], hi[2], 0.0f);
-    }
-    __syncwarp();
-    if (in_seg) {
-        const float4 a = x[lane].lo, b = x[lane].hi;
-        lo[0] = a.x;
-        lo[1] = a.y;
-        lo[2] = a.z;
-        id = __float_as_uint(a.w);
-        hi[0] = b.x;
-        hi[1] = b.y;
-        hi[2] = b.z;
-    }
-    __syncwarp();
-}
-
-// Build the subtree rooted at a node of n0 <= 32 objects. Lane i < n0 holds
-// object i of the node's range (starting at global position `base`).
-// Writes every node of the subtree and the permutation entries of its range.
-__device__ void warp_build_subtree(float lo[3], float hi[3], uint32_t id, uint32_t n0, uint32_t base,
-                                   uint32_t slot0, uint32_t pair0, uint32_t depth0, uint32_t nbase,
-                                   uint32_t tbase, const float* bounds0, const Params& P, const Out& O,
-                                   XRec* xchg) {
-    const uint32_t lane = threadIdx.x & 31u;
-    // Pending-node stack, entry k held by lane k.
-    uint32_t st_sn = 0, st_slot = 0, st_pair = 0, st_depth = 0;
-    float st_b[6];
-    if (lane == 0) {
-        st_sn = n0 << 8;
-        st_slot = slot0;
-        st_pair = pair0;
-        st_depth = depth0;
-        for (int i = 0; i < 6; ++i) st_b[i] = bounds0[i];
-    }
-    int top = 1;
-    uint32_t max_split_depth = 0;
-    bool any_split = false;
-    uint32_t n_median = 0, n_holes = 0, n_capped = 0;
-
-    while (top > 0) {
-        --top;
-        const uint32_t sn = __shfl_sync(kFull, st_sn, top);
-        const uint32_t s = sn & 0xFFu, n = sn >> 8;
-        const uint32_t slot = __shfl_sync(kFull, st_slot, top);
-        const uint32_t pair = __shfl_sync(kFull, st_pair, top);
-        const uint32_t depth = __shfl_sync(kFull, st_depth, top);
-        float nb[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) nb[i] = __shfl_sync(kFull, st_b[i], top);
-
-        const bool in_seg = lane >= s && lane < s + n;
-        bool leaf = n <= 1u || depth == P.max_depth ||
-                    (n <= P.max_leaf && n < 2u * P.min_leaf);  // bvh/src/lib.rs:548, 556
-        uint32_t n_lt = 0;
-        Cand win;
-        bool adaptive = false;  // adaptive: c < thr; binned: bin < idx; median: position
-        bool median = false;
-        uint32_t win_axis = 0, win_idx = 0;
-        uint32_t mybins = 0;  // this lane's bin per axis (binned sweep), 8 bits each
-
-        if (!leaf) {
-            float c[3], cmn[3], cmx[3], ext[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) c[a] = center_of(lo[a], hi[a]);
-            // centroid bounds (bvh/src/lib.rs:499-509)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                cmn[a] = funkey(__reduce_min_sync(kFull, in_seg ? fkey(c[a]) : kKeyPosInf));
-                cmx[a] = funkey(__reduce_max_sync(kFull, in_seg ? fkey(c[a]) : kKeyNegInf));
-                ext[a] = __fsub_rn(cmx[a], cmn[a]);
-            }
-            const float sa_p = surface_area6(nb);
-            Cand best;
-            best.key = ~0ull;
-            adaptive = n <= P.adaptive_max_n;
-            if (adaptive) {
-                // adaptive_sweep, bvh/src/lib.rs:392-442
-                const bool exact = n < 8u;
-                const uint32_t steps =
-                    exact ? n : (P.adaptive_steps ? P.adaptive_steps : min(max(n, 8u), 32u));
-                const bool cand = exact ? in_seg : lane < steps;
-                const uint32_t cidx = exact ? lane - s : lane;
-                float thr[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float step = __fdiv_rn(ext[a], __uint2float_rn(steps));
-                    thr[a] = exact ? c[a] : adaptive_threshold(cmn[a], step, lane);
-                }
-                float blt[3][6], bgt[3][6];
-                uint32_t nlt[3] = {0, 0, 0};
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    box_empty(blt[a]);
-                    box_empty(bgt[a]);
-                }
-                for (uint32_t j = s; j < s + n; ++j) {
-                    const float jl0 = __shfl_sync(kFull, lo[0], j), jl1 = __shfl_sync(kFull, lo[1], j),
-                                jl2 = __shfl_sync(kFull, lo[2], j);
-                    const float jh0 = __shfl_sync(kFull, hi[0], j), jh1 = __shfl_sync(kFull, hi[1], j),
-                                jh2 = __shfl_sync(kFull, hi[2], j);
-                    const float jc[3] = {center_of(jl0, jh0), center_of(jl1, jh1), center_of(jl2, jh2)};
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        if (jc[a] < thr[a]) {  // bvh/src/lib.rs:308
-                            box_grow(blt[a], jl0, jl1, jl2, jh0, jh1, jh2);
-                            nlt[a]++;
-                        } else {
-                            box_grow(bgt[a], jl0, jl1, jl2, jh0, jh1, jh2);
-                        }
-                    }
-                }
-                if (cand) {
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const uint32_t ng = n - nlt[a];
-                        if (nlt[a] >= P.min_leaf && ng >= P.min_leaf) {  // :407
-                            const float cost = split_cost(surface_area6(blt[a]), surface_area6(bgt[a]),
-                                                          sa_p, nlt[a], ng);
-                            const uint64_t k = cand_key(cost, a, cidx);
-                            if (k < best.key) {
-                                best.key = k;
-                                best.n_lt = nlt[a];
-                                best.thr = thr[a];
-                                for (int i = 0; i < 6; ++i) {
-                                    best.lt[i] = blt[a][i];
-                                    best.gt[i] = bgt[a][i];
-                                }
-                            }
-                        }
-                    }
-                }
-            } else {
-                // binned_sweep, bvh/src/lib.rs:331-389
-                const uint32_t bins = P.bins ? P.bins : min(max(n, 16u), 32u);
-                bool axis_ok[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    axis_ok[a] = !(ext[a] == 0.0f);  // :339
-                    const uint32_t b = axis_ok[a] ? bin_of(c[a], cmn[a], ext[a], bins) : 0u;
-                    mybins |= b << (8 * a);
-                }
-                uint32_t cnt[3] = {0, 0, 0};
-                float box[3][6];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) box_empty(box[a]);
-                for (uint32_t j = s; j < s + n; ++j) {
-                    const float jl0 = __shfl_sync(kFull, lo[0], j), jl1 = __shfl_sync(kFull, lo[1], j),
-                                jl2 = __shfl_sync(kFull, lo[2], j);
-                    const float jh0 = __shfl_sync(kFull, hi[0], j), jh1 = __shfl_sync(kFull, hi[1], j),
-                                jh2 = __shfl_sync(kFull, hi[2], j);
-                    const uint32_t jb = __shfl_sync(kFull, mybins, j);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        if (((jb >> (8 * a)) & 0xFFu) == lane) {
-                            box_grow(box[a], jl0, jl1, jl2, jh0, jh1, jh2);
-                            cnt[a]++;
-                        }
-                    }
-                }
-                binned_candidates(cnt, box, axis_ok, bins, n, sa_p, P, lane, best);
-            }
-            const uint64_t wk = warp_min_key(best.key);
-            const uint32_t wlo = static_cast<uint32_t>(wk);
-            if (wlo == kNoKey) {
-                if (n > P.max_leaf) {
-                    median = true;  // bvh/src/lib.rs:527-531
-                } else {
-                    leaf = true;  // :576-579
-                }
-            } else {
-                win_axis = (wlo >> 8) & 3u;
-                win_idx = wlo & 0xFFu;
-                const uint32_t src = (adaptive && n < 8u) ? s + win_idx : win_idx;
-                win = best;
-                shfl_cand(win, src);
-                const float cost = funkey(static_cast<uint32_t>(wk >> 32));
-                if (n <= P.max_leaf && cost >= leaf_cost(n)) leaf = true;  // :583
-                n_lt = win.n_lt;
-            }
-
-            if (median) {
-                // median_split on axes 0, 1, 2 in turn over the same list
-                // (bvh/src/lib.rs:444-491, 528-530); keep the first minimum.
-                const uint32_t m = n / 2u;
-                uint32_t best_ck = 0;
-                for (uint32_t a = 0; a < 3; ++a) {
-                    const float ca = center_of(sel3(lo, a), sel3(hi, a));
-                    const uint32_t key = fkey(ca);
-                    uint32_t rank = 0;
-                    for (uint32_t j = s; j < s + n; ++j) {
-                        const uint32_t kj = __shfl_sync(kFull, key, j);
-                        rank += (kj < key || (kj == key && j < lane)) ? 1u : 0u;
-                    }
-                    const bool pr = in_seg && rank < m;
-                    warp_stable_permute(in_seg, pr, s, m, lane, lo, hi, id, xchg);
-                    float blt[6], bgt[6];
-                    const bool in_lt = lane >= s && lane < s + m;
-                    const bool in_gt = lane >= s + m && lane < s + n;
-                    warp_box_union(in_lt, lo, hi, blt);
-                    warp_box_union(in_gt, lo, hi, bgt);
-                    const float cost =
-                        split_cost(surface_area6(blt), surface_area6(bgt), sa_p, m, n - m);
-                    const uint32_t ck = fkey(cost);
-                    if (a == 0 || ck < best_ck) {
-                        best_ck = ck;
-                        win_axis = a;
-                        for (int i = 0; i < 6; ++i) {
-                            win.lt[i] = blt[i];
-                            win.gt[i] = bgt[i];
-                        }
-                    }
-                }
-                n_lt = m;
-                n_median++;
-            }
-        }
-
-        if (leaf) {
-            warp_store_node(O, nbase + slot, nb, base + s - tbase, n, 0u, lane);
-            if (in_seg) O.perm[base + lane] = id;
-            if (n > 1u) {
-                n_holes++;
-                if (depth == P.max_depth) n_capped++;
-            }
-            continue;
-        }
-
-        // partition (bvh/src/lib.rs:597-612), stable
-        float c[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) c[a] = center_of(lo[a], hi[a]);
-        bool pred;
-        if (median) {
-            pred = lane < s + n_lt;  // Exact { index }: split at the position
-        } else if (adaptive) {
-            const float cw = win_axis == 0 ? c[0] : (win_axis == 1 ? c[1] : c[2]);
-            pred = cw < win.thr;
-        } else {
-            pred = ((mybins >> (8 * win_axis)) & 0xFFu) < win_idx;
-        }
-        const uint32_t ltm = __ballot_sync(kFull, in_seg && pred);
-        if (static_cast<uint32_t>(__popc(ltm)) != n_lt) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
-        // containment of centroids in child bounds (bvh/src/lib.rs:637-646)
-        const bool ok = !in_seg || box_contains2(win.lt, win.gt, pred, c[0], c[1], c[2]);
-        if (__ballot_sync(kFull, !ok)) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
-        warp_store_node(O, nbase + slot, nb, base + s - tbase, n, pair, lane);
-        if (!median) warp_stable_permute(in_seg, pred, s, n_lt, lane, lo, hi, id, xchg);
-
-        any_split = true;
-        max_split_depth = max(max_split_depth, depth);
-        const uint32_t n_gt = n - n_lt;
-        // push lt, then gt (gt is visited first; order does not change slots)
-        if (lane == static_cast<uint32_t>(top)) {
-            st_sn = s | (n_lt << 8);
-            st_slot = pair + 1u;
-            st_pair = pair + 2u * n_gt;
-            st_depth = depth + 1u;
-            for (int i = 0; i < 6; ++i) st_b[i] = win.lt[i];
-        }
-        if (lane == static_cast<uint32_t>(top + 1)) {
-            st_sn = (s + n_lt) | (n_gt << 8);
-            st_slot = pair;
-            st_pair = pair + 2u;
-            st_depth = depth + 1u;
-            for (int i = 0; i < 6; ++i) st_b[i] = win.gt[i];
-        }
-        top += 2;
-    }
-    if (lane == 0) {
-        if (any_split) atomicMax(&O.ctr->height, max_split_depth);
-        if (n_median) atomicAdd(&O.ctr->median_splits, n_median);
-        if (n_holes) atomicAdd(&O.ctr->holes, n_holes);
-        if (n_capped) atomicAdd(&O.ctr->depth_capped, n_capped);
-    }
-}
-
 // Segmented reductions over contiguous lane ranges [s, end): shuffle-down
 // tree bounded by the segment end, then a broadcast from the segment's first
-// lane. Every lane takes part with full masks (per-segment masks in one
+// lane; maxn (warp-uniform) is the longest segment, past which no step adds
+// anything. Every lane takes part with full masks (per-segment masks in one
 // warp serialize: one pass per distinct mask).
-__device__ __forceinline__ uint32_t seg_min(uint32_t v, uint32_t lane, uint32_t s, uint32_t end) {
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
+__device__ __forceinline__ uint32_t seg_min(uint32_t v, uint32_t lane, uint32_t s, uint32_t end, uint32_t maxn) {
+    for (uint32_t d = 1; d < maxn; d <<= 1) {
         const uint32_t u = __shfl_down_sync(kFull, v, d);
         if (lane + d < end) v = min(v, u);
     }
     return __shfl_sync(kFull, v, s);
 }
 
-__device__ __forceinline__ uint32_t seg_max(uint32_t v, uint32_t lane, uint32_t s, uint32_t end) {
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
+__device__ __forceinline__ uint32_t seg_max(uint32_t v, uint32_t lane, uint32_t s, uint32_t end, uint32_t maxn) {
+    for (uint32_t d = 1; d < maxn; d <<= 1) {
         const uint32_t u = __shfl_down_sync(kFull, v, d);
         if (lane + d < end) v = max(v, u);
     }
@@ -640,10 +334,9 @@ __device__ __forceinline__ uint32_t seg_max(uint32_t v, uint32_t lane, uint32_t 
 }
 
 // Lexicographic (hi, lo) minimum over the segment.
-__device__ __forceinline__ void seg_min2(uint32_t& hi, uint32_t& lo, uint32_t lane, uint32_t s,
-                                         uint32_t end) {
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
+__device__ __forceinline__ void seg_min2(uint32_t& hi, uint32_t& lo, uint32_t lane, uint32_t s, uint32_t end,
+                                         uint32_t maxn) {
+    for (uint32_t d = 1; d < maxn; d <<= 1) {
         const uint32_t uh = __shfl_down_sync(kFull, hi, d);
         const uint32_t ul = __shfl_down_sync(kFull, lo, d);
         if (lane + d < end && (uh < hi || (uh == hi && ul < lo))) {
@@ -686,271 +379,547 @@ __device__ __forceinline__ void lane_store_node(const Out& o, uint32_t slot, con
     o.used[slot] = 1;
 }
 
-// Moves this lane's object to lane `dst` (a permutation of the warp).
-__device__ __forceinline__ void warp_exchange(uint32_t dst, uint32_t lane, float* lo, float* hi,
-                                              uint32_t& id, XRec* x) {
-    x[dst].lo = make_float4(lo[0], lo[1], lo[2], __uint_as_float(id));
-    x[dst].hi = make_float4(hi[0], hi[1], hi[2], 0.0f);
-    __syncwarp();
-    const float4 a = x[lane].lo, b = x[lane].hi;
-    lo[0] = a.x;
-    lo[1] = a.y;
-    lo[2] = a.z;
-    id = __float_as_uint(a.w);
-    hi[0] = b.x;
-    hi[1] = b.y;
-    hi[2] = b.z;
-    __syncwarp();
+// A warp's tables of one subtree of n0 <= 32 objects.
+//
+// Every object set the builder looks at is a set of the subtree's n0 objects,
+// kept as masks over nine orders: for each of the six box coordinates, bit b
+// stands for the object at place b of that coordinate's order (its lower
+// bounds descending, its upper bounds ascending), so the union box's
+// coordinate is the value at the mask's highest bit, which lane b holds: one
+// find-leading-one and one shuffle instead of a min/max over the set. Orders
+// 6..8 are the centroids' on each axis, ascending. The objects left of a
+// threshold on axis a are the first m of its order, for whatever node of the
+// subtree: pm[a][q][m - 1] holds them as bits of order q, made once, and a
+// node's left side is that mask and the node's own.
+constexpr uint32_t kOrders = 9;
+
+struct alignas(16) SubtreeSmem {
+    uint32_t head[32];  // (reads for m = 0, whose value is not used, fall here)
+    uint32_t pm[3][kOrders][32];  // 32 words a plane: lanes with different m read different banks
+    uint32_t rt[32];   // by place on axis 0: the object's bit in each coordinate's order (5 bits each)
+    uint32_t ids[32];  // by place on axis 0: the object's id
+    uint32_t x[32];    // exchange space
+};
+
+// What a lane holds of the tables: coordinate q's value at bit `lane`, and the
+// centroid on axis a at place `lane` of its order (NaN past the last).
+struct SubtreeRegs {
+    float val[6], cen[3];
+};
+
+// Highest set bit of a mask; -1 for an empty one (a shuffle reads lane 31
+// then, and the value is not used).
+__device__ __forceinline__ int top_bit(uint32_t m) {
+    int r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(m));
+    return r;
 }
 
-// Level-synchronous form of warp_build_subtree: every node of one depth of
-// the subtree is evaluated at the same time, each on its own lane range
-// (segment), with segmented warp reductions. Valid when every node of the
-// subtree uses the adaptive sweep with one threshold per object: the
-// reference profile (steps = len.clamp(8,32) = len for 8 <= len <= 32, one
-// centroid per object below 8; bvh/src/lib.rs:417-437).
-__device__ void warp_build_subtree_levels(float lo[3], float hi[3], uint32_t id, uint32_t n0,
-                                          uint32_t base, uint32_t slot0, uint32_t pair0,
-                                          uint32_t depth0, uint32_t nbase, uint32_t tbase,
-                                          const float* bounds0, const Params& P, const Out& O,
-                                          XRec* xchg) {
+__device__ __forceinline__ bool leaf_rule(uint32_t n, uint32_t depth, const Params& P) {
+    return n <= 1u || depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf);  // bvh/src/lib.rs:548, 556
+}
+
+// Split profiles other than the reference's own (every node of <= 32 objects
+// adaptive, with one threshold per object: steps = len.clamp(8,32) = len for
+// 8 <= len <= 32, one centroid per object below 8; bvh/src/lib.rs:417-437).
+__host__ __device__ __forceinline__ bool subtree_general(const Params& P) {
+    return P.adaptive_steps != 0u || P.adaptive_max_n != kSmallMax;
+}
+
+// Fills T for the objects of lanes 0 .. n0-1 (lo, hi, id; 2 <= n0 <= 32) and
+// returns this lane's object word: its place on axis a at bits 5a, and the
+// number of objects with a lower centroid on a at bits 15 + 5a.
+__device__ __forceinline__ uint32_t subtree_tables(const float* lo, const float* hi, uint32_t id, uint32_t n0,
+                                                   uint32_t lane, SubtreeSmem& T, SubtreeRegs& R) {
+    static_assert(sizeof(T.pm) >= 32 * 48 + 9 * 128, "the sort space fits in the prefix masks' space");
+    const uint32_t below = (1u << lane) - 1u;
+    // sort keys: NaN coordinates rank where fminf / fmaxf ignore them, NaN
+    // centroids last
+    float v[9], c[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        c[a] = center_of(lo[a], hi[a]);
+        v[a] = fminf(lo[a], __int_as_float(0x7F800000));
+        v[3 + a] = fmaxf(hi[a], __int_as_float(0xFF800000));
+        v[6 + a] = fminf(c[a], __int_as_float(0x7F800000));
+    }
+    float4* keys = reinterpret_cast<float4*>(&T.pm[0][0][0]);
+    uint32_t* sp = &T.pm[0][0][0] + 32 * 12;  // 9 x 32 words
+    keys[3 * lane] = make_float4(v[0], v[1], v[2], v[3]);
+    keys[3 * lane + 1] = make_float4(v[4], v[5], v[6], v[7]);
+    keys[3 * lane + 2] = make_float4(v[8], 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (uint32_t q = 0; q < 9; ++q) sp[32u * q + lane] = 0u;
+    __syncwarp();
+    uint32_t r[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) r[q] = 0;
+#pragma unroll 4
+    for (uint32_t j = 0; j < n0; ++j) {  // one address per step: broadcast loads
+        const float4 k0 = keys[3 * j], k1 = keys[3 * j + 1];
+        const float k2 = keys[3 * j + 2].x;
+        r[0] += k0.x < v[0] ? 1u : 0u;
+        r[1] += k0.y < v[1] ? 1u : 0u;
+        r[2] += k0.z < v[2] ? 1u : 0u;
+        r[3] += k0.w < v[3] ? 1u : 0u;
+        r[4] += k1.x < v[4] ? 1u : 0u;
+        r[5] += k1.y < v[5] ? 1u : 0u;
+        r[6] += k1.z < v[6] ? 1u : 0u;
+        r[7] += k1.w < v[7] ? 1u : 0u;
+        r[8] += k2 < v[8] ? 1u : 0u;
+    }
+    // equal keys take consecutive places in lane order
+    const bool mine = lane < n0;
+    if (mine) {
+#pragma unroll
+        for (uint32_t q = 0; q < 9; ++q) atomicOr(&sp[32u * q + r[q]], 1u << lane);
+    }
+    __syncwarp();
+    uint32_t word = 0, bits = 0, place[9];
+#pragma unroll
+    for (uint32_t q = 0; q < 9; ++q) place[q] = r[q] + (mine ? __popc(sp[32u * q + r[q]] & below) : 0u);
+    __syncwarp();
+    float* rows = reinterpret_cast<float*>(sp);
+    if (mine) {
+#pragma unroll
+        for (uint32_t q = 0; q < 6; ++q) {
+            const uint32_t b = q < 3 ? 31u - place[q] : place[q];
+            rows[32u * q + b] = v[q];
+            bits |= b << (5u * q);
+        }
+#pragma unroll
+        for (uint32_t a = 0; a < 3; ++a) {
+            rows[32u * (6u + a) + place[6 + a]] = c[a];
+            // (a NaN centroid is below no threshold and no threshold itself)
+            word |= place[6 + a] << (5u * a) | (c[a] == c[a] ? r[6 + a] : 0u) << (15u + 5u * a);
+        }
+        T.rt[place[6]] = bits;
+        T.ids[place[6]] = id;
+    } else {
+#pragma unroll
+        for (uint32_t a = 0; a < 3; ++a) rows[32u * (6u + a) + lane] = __int_as_float(0x7FFFFFFF);
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t q = 0; q < 6; ++q) R.val[q] = rows[32u * q + lane];
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) R.cen[a] = rows[32u * (6u + a) + lane];
+    // prefix masks: lane p takes the object at place p of the axis's order
+    uint32_t* xw = &T.pm[0][0][0];  // the keys' space: bits and words by place
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        if (mine) {
+            xw[64u * a + place[6 + a]] = bits;
+            xw[64u * a + 32u + place[6 + a]] = word;
+        }
+    }
+    __syncwarp();
+    uint32_t pb[3], pw[3];
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        pb[a] = xw[64u * a + lane];
+        pw[a] = xw[64u * a + 32u + lane];
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        uint32_t w[kOrders];
+#pragma unroll
+        for (uint32_t q = 0; q < kOrders; ++q) {
+            const uint32_t b = q < 6 ? pb[a] >> (5u * q) : pw[a] >> (5u * (q - 6u));
+            w[q] = mine ? 1u << (b & 31u) : 0u;
+        }
+#pragma unroll
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+#pragma unroll
+            for (uint32_t q = 0; q < kOrders; ++q) {
+                if (q == 6u + a) continue;
+                const uint32_t u = __shfl_up_sync(kFull, w[q], d);
+                if (lane >= d) w[q] |= u;
+            }
+        }
+        w[6 + a] = mine ? below | (1u << lane) : (1u << n0) - 1u;  // the axis's own order
+#pragma unroll
+        for (uint32_t q = 0; q < kOrders; ++q) {
+            T.pm[a][q][lane] = w[q];
+        }
+    }
+    __syncwarp();
+    return word;
+}
+
+// The candidate of an object (place `place`, centroid c, predecessor's
+// centroid prev) on an axis of a node that takes evenly spaced thresholds
+// (n >= 8 adaptive) or bins: the split whose gt side starts at this object in
+// the node's centroid order, with the lowest threshold or bin index that makes
+// this split. False when no threshold falls between the object and its
+// predecessor. The sets {c < threshold i} and {bin < i} are prefixes of the
+// centroid order (threshold and bin are monotone), so these are all the
+// different splits of the sweep, each with its first index.
+__device__ __forceinline__ bool ordered_candidate(float c, float prev, float cmin, float cmax, uint32_t n,
+                                                  bool adaptive, const Params& P, uint32_t& idx) {
+    const float ext = __fsub_rn(cmax, cmin);
+    if (adaptive) {  // bvh/src/lib.rs:428-441: the first threshold above prev, if not above c
+        const uint32_t steps = P.adaptive_steps ? P.adaptive_steps : n;
+        const float step = __fdiv_rn(ext, __uint2float_rn(steps));
+        uint32_t lo = 0, hi = steps;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (prev < adaptive_threshold(cmin, step, mid))
+                hi = mid;
+            else
+                lo = mid + 1u;
+        }
+        idx = lo;
+        return lo < steps && !(c < adaptive_threshold(cmin, step, lo));
+    }
+    if (ext == 0.0f) return false;  // bvh/src/lib.rs:339
+    const uint32_t bins = P.bins ? P.bins : min(max(n, 16u), 32u);
+    const uint32_t b = bin_of(prev, cmin, ext, bins);
+    idx = b + 1u;
+    return b < bin_of(c, cmin, ext, bins);
+}
+
+struct MedianIo {
+    SubtreeRegs regs;
+    float nb[6];             // in: the node's box; out: the lane's half's
+    uint32_t node[kOrders];  // out: the lane's half as masks
+    uint32_t word;           // in and out: the lane's object
+};
+
+// median_split (bvh/src/lib.rs:444-491, 528-530) of the segments whose lanes
+// have `odd`: on axes 0, 1, 2 in turn over the same list, stable; the halves
+// are those of the final (axis-2) order, their boxes the cheapest axis's. All
+// lanes take part. Rare: kept out of line, so that its registers are not the
+// main loop's.
+__device__ __forceinline__ void median_segments(bool odd, uint32_t s, uint32_t n, uint32_t m, uint32_t ss, uint32_t se,
+                                             uint32_t maxn, SubtreeSmem& T, MedianIo& io) {
+    const SubtreeRegs R = io.regs;
+    const NodeArea area(io.nb);
+    uint32_t word = io.word;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
+    const uint32_t half = n / 2u;
+    float wb[6];
+    uint32_t best_ck = 0;
+#pragma unroll 1
+    for (uint32_t a = 0; a < 3; ++a) {
+        const float cen = a == 0 ? R.cen[0] : (a == 1 ? R.cen[1] : R.cen[2]);
+        const uint32_t key = fkey(__shfl_sync(kFull, cen, (word >> (5u * a)) & 31u));
+        uint32_t rank = 0;
+        for (uint32_t r = 0; r < maxn; ++r) {
+            const bool use = odd && r < n;
+            const uint32_t kj = __shfl_sync(kFull, key, use ? s + r : lane);
+            if (use) rank += (kj < key || (kj == key && s + r < lane)) ? 1u : 0u;
+        }
+        const uint32_t lm = __ballot_sync(kFull, odd && rank < half) & m;
+        T.x[odd ? (rank < half ? s + __popc(lm & below) : s + half + __popc(m & ~lm & below)) : lane] = word;
+        __syncwarp();
+        word = T.x[lane];
+        __syncwarp();
+        const uint32_t bits = T.rt[word & 31u];
+        const bool in_lt = odd && lane < s + half, in_gt = odd && lane >= s + half;
+        float l6[6], g6[6];
+#pragma unroll
+        for (uint32_t i = 0; i < 6; ++i) {
+            const uint32_t k = fkey(__shfl_sync(kFull, R.val[i], (bits >> (5u * i)) & 31u));
+            if (i < 3) {
+                l6[i] = funkey(seg_min(in_lt ? k : kKeyPosInf, lane, ss, se, maxn));
+                g6[i] = funkey(seg_min(in_gt ? k : kKeyPosInf, lane, ss, se, maxn));
+            } else {
+                l6[i] = funkey(seg_max(in_lt ? k : kKeyNegInf, lane, ss, se, maxn));
+                g6[i] = funkey(seg_max(in_gt ? k : kKeyNegInf, lane, ss, se, maxn));
+            }
+        }
+        const uint32_t ck = fkey(area.split_cost(surface_area6(l6), surface_area6(g6), half, n - half));
+        if (a == 0u || ck < best_ck) {
+            best_ck = ck;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) wb[i] = in_lt ? l6[i] : g6[i];
+        }
+    }
+    const uint32_t bits = T.rt[word & 31u];
+    uint32_t hm[kOrders];
+#pragma unroll
+    for (uint32_t q = 0; q < kOrders; ++q) hm[q] = 0;
+    for (uint32_t r = 0; r < maxn; ++r) {
+        const uint32_t src = odd && r < n ? s + r : lane;
+        const uint32_t bj = __shfl_sync(kFull, bits, src), wj = __shfl_sync(kFull, word, src);
+        if (odd && r < n && (r < half) == (lane < s + half)) {
+#pragma unroll
+            for (uint32_t q = 0; q < kOrders; ++q)
+                hm[q] |= 1u << ((q < 6u ? bj >> (5u * q) : wj >> (5u * (q - 6u))) & 31u);
+        }
+    }
+    io.word = word;
+#pragma unroll
+    for (uint32_t q = 0; q < kOrders; ++q) io.node[q] = hm[q];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) io.nb[i] = wb[i];
+}
+
+// Builds the subtree rooted at a node of n0 <= 32 objects. Lane i < n0 holds
+// object i of the node's range (starting at global position `base`). Writes
+// every node of the subtree and the permutation entries of its range.
+// kGeneral: any split profile (subtree_general).
+//
+// Every node of one depth is evaluated at the same time, each on its own lane
+// range (segment): a lane holds the candidate of its object or threshold on
+// each axis, with both sides' boxes read from the tables (SubtreeSmem).
+// What bounds it: issued instructions (75-80% of the issue slots). A merge of
+// every object into every candidate, O(n^2) per node, took 465M warp
+// instructions on the level-8 icosphere's 59,272 subtrees (22 objects, 5.1
+// depths each): 0.544 ms. With the orders sorted once per subtree (about 1,500
+// instructions) and 36 mask-and-shuffle reads per lane and depth (700-900
+// instructions a depth) it is 329M: 0.386 ms. The general profiles use the same
+// tables in place of a depth-first form with one node at a time: 65,536 random
+// triangles at 16 bins, 0.325 -> 0.047 ms; 16.8M mixed triangles, 8.3 -> 5.3 ms.
+template <bool kGeneral>
+__device__ void warp_build_subtree(const float* lo, const float* hi, uint32_t id, uint32_t n0, uint32_t base,
+                                   uint32_t slot0, uint32_t pair0, uint32_t depth0, uint32_t nbase, uint32_t tbase,
+                                   const float* bounds0, const Params& P, const Out& O, SubtreeSmem& T) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
+    if (leaf_rule(n0, depth0, P)) {  // warp-uniform; the queued roots split
+        if (lane == 0) {
+            lane_store_node(O, nbase + slot0, bounds0, base - tbase, n0, 0u);
+            if (n0 > 1u) {
+                atomicAdd(&O.ctr->holes, 1u);
+                if (depth0 == P.max_depth) atomicAdd(&O.ctr->depth_capped, 1u);
+            }
+        }
+        if (lane < n0) O.perm[base + lane] = id;
+        return;
+    }
+    __syncwarp();  // the previous subtree's table reads are done
+    SubtreeRegs R;
+    uint32_t word = subtree_tables(lo, hi, id, n0, lane, T, R);
     uint32_t s = 0, n = n0, slot = slot0, pair = pair0, depth = depth0;
+    bool live = lane < n0;
+    uint32_t node[kOrders];  // the segment's objects as a mask of each order
+#pragma unroll
+    for (uint32_t q = 0; q < kOrders; ++q) node[q] = live ? T.pm[0][q][31] : 0u;
     float nb[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) nb[i] = bounds0[i];
-    bool live = lane < n0;
     uint32_t hmax = 0, n_median = 0, n_holes = 0, n_capped = 0;
-    bool any_split = false;
+    if (lane == 0) lane_store_node(O, nbase + slot, nb, base - tbase, n, pair);
 
     while (__any_sync(kFull, live)) {
         const uint32_t m = live ? seg_mask(s, n) : (1u << lane);
         const uint32_t ss = live ? s : lane, se = live ? s + n : lane + 1u;  // reduction range
-        const bool leader = live && lane == s;
-        bool leaf = n <= 1u || depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf);
-        const bool work = live && !leaf;
-        float c[3];
+        const uint32_t maxn = __reduce_max_sync(kFull, live ? n : 0u);
+        const NodeArea area(nb);
+        // this lane's candidate per axis: the lt side's size in the axis's
+        // order. Below 8 objects every object's own centroid is a threshold
+        uint32_t cut[3], idx[3] = {lane, lane, lane};
+        bool ok[3] = {live, live, live};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) c[a] = center_of(lo[a], hi[a]);
-        const float sa_p = surface_area6(nb);
-        const bool exact = n < 8u;
-        const uint32_t k = lane - s;
-        // thresholds: below 8 objects each object's own centroid; else the
-        // adaptive steps over the segment's centroid bounds
-        // (bvh/src/lib.rs:499-509), which only such segments need (the
-        // warp skips the reductions when it has none)
-        float thr[3] = {c[0], c[1], c[2]};
-        if (__any_sync(kFull, work && !exact)) {
+        for (int a = 0; a < 3; ++a) cut[a] = (word >> (15 + 5 * a)) & 31u;
+        if constexpr (kGeneral) {
+            const bool adaptive = n <= P.adaptive_max_n;
+            const bool ordered = live && !(adaptive && n < 8u);
+            if (__any_sync(kFull, ordered)) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float cmn = funkey(seg_min(work ? fkey(c[a]) : kKeyPosInf, lane, ss, se));
-                const float cmx = funkey(seg_max(work ? fkey(c[a]) : kKeyNegInf, lane, ss, se));
-                if (!exact) {
-                    const float step = __fdiv_rn(__fsub_rn(cmx, cmn), __uint2float_rn(n));
-                    thr[a] = adaptive_threshold(cmn, step, k);
-                }
-            }
-        }
-        float blt[3][6], bgt[3][6];
-        uint32_t nlt[3] = {0, 0, 0};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            box_empty(blt[a]);
-            box_empty(bgt[a]);
-        }
-        const uint32_t maxn = __reduce_max_sync(kFull, work ? n : 0u);
-        // every lane's object in shared memory, with its x and y centroids in
-        // the spare words; the lanes of a segment read its objects in turn
-        // (one address per segment: broadcast loads)
-        xchg[lane].lo = make_float4(lo[0], lo[1], lo[2], c[0]);
-        xchg[lane].hi = make_float4(hi[0], hi[1], hi[2], c[1]);
-        __syncwarp();
-        for (uint32_t r = 0; r < maxn; ++r) {
-            if (!(work && r < n)) continue;  // lanes past their segment's objects merge nothing
-            const float4 ja = xchg[s + r].lo, jb = xchg[s + r].hi;
-            const float jl0 = ja.x, jl1 = ja.y, jl2 = ja.z, jh0 = jb.x, jh1 = jb.y, jh2 = jb.z;
-            const float jc[3] = {ja.w, jb.w, center_of(jl2, jh2)};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (jc[a] < thr[a]) {  // bvh/src/lib.rs:308
-                    blt[a][0] = fminf(blt[a][0], jl0);
-                    blt[a][1] = fminf(blt[a][1], jl1);
-                    blt[a][2] = fminf(blt[a][2], jl2);
-                    blt[a][3] = fmaxf(blt[a][3], jh0);
-                    blt[a][4] = fmaxf(blt[a][4], jh1);
-                    blt[a][5] = fmaxf(blt[a][5], jh2);
-                    nlt[a]++;
-                } else {
-                    bgt[a][0] = fminf(bgt[a][0], jl0);
-                    bgt[a][1] = fminf(bgt[a][1], jl1);
-                    bgt[a][2] = fminf(bgt[a][2], jl2);
-                    bgt[a][3] = fmaxf(bgt[a][3], jh0);
-                    bgt[a][4] = fmaxf(bgt[a][4], jh1);
-                    bgt[a][5] = fmaxf(bgt[a][5], jh2);
-                }
-            }
-        }
-        __syncwarp();  // reads of xchg done before the exchanges below rewrite it
-        Cand best;
-        best.key = ~0ull;
-        best.n_lt = 0;
-        best.thr = 0.0f;
-        if (work) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const uint32_t ng = n - nlt[a];
-                if (nlt[a] >= P.min_leaf && ng >= P.min_leaf) {  // :407
-                    const float cost =
-                        split_cost(surface_area6(blt[a]), surface_area6(bgt[a]), sa_p, nlt[a], ng);
-                    const uint64_t key = cand_key(cost, a, k);
-                    if (key < best.key) {
-                        best.key = key;
-                        best.n_lt = nlt[a];
-                        best.thr = thr[a];
-                        for (int i = 0; i < 6; ++i) {
-                            best.lt[i] = blt[a][i];
-                            best.gt[i] = bgt[a][i];
-                        }
+                for (uint32_t a = 0; a < 3; ++a) {
+                    const uint32_t place = (word >> (5u * a)) & 31u;
+                    const uint32_t before = node[6 + a] & ((1u << place) - 1u);
+                    const float c = __shfl_sync(kFull, R.cen[a], place);
+                    const float prev = __shfl_sync(kFull, R.cen[a], top_bit(before));
+                    const float cmin = __shfl_sync(kFull, R.cen[a], __ffs(node[6 + a]) - 1);
+                    const float cmax = __shfl_sync(kFull, R.cen[a], top_bit(node[6 + a]));
+                    if (ordered) {
+                        cut[a] = place;
+                        ok[a] = before != 0u && ordered_candidate(c, prev, cmin, cmax, n, adaptive, P, idx[a]);
                     }
                 }
             }
+        } else if (maxn >= 8u) {
+            // adaptive steps over the segment's centroid bounds
+            // (bvh/src/lib.rs:428-441, 499-509), one threshold per lane; the
+            // lt side's size by binary search in the axis's order
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float cmin = __shfl_sync(kFull, R.cen[a], __ffs(node[6 + a]) - 1);
+                const float cmax = __shfl_sync(kFull, R.cen[a], top_bit(node[6 + a]));
+                // (1: lanes of other nodes, whose step is not used)
+                const float ext = live && n >= 8u ? __fsub_rn(cmax, cmin) : 1.0f;
+                const float step = __fdiv_rn(ext, __uint2float_rn(n));
+                const float thr = adaptive_threshold(cmin, step, lane - s);
+                uint32_t p = 0;
+#pragma unroll
+                for (uint32_t h = 16; h > 0; h >>= 1)
+                    if (__shfl_sync(kFull, R.cen[a], p + h - 1u) < thr) p += h;
+                if (__shfl_sync(kFull, R.cen[a], p) < thr) ++p;
+                if (n >= 8u) cut[a] = p;
+            }
         }
-        // first minimum per segment: (cost, axis, threshold index)
-        uint32_t mh = static_cast<uint32_t>(best.key >> 32);
-        uint32_t ml = static_cast<uint32_t>(best.key);
-        seg_min2(mh, ml, lane, ss, se);
-        const bool found = work && ml != kNoKey;
-        bool median = false;
-        uint32_t axis = 0, n_lt = 0;
-        Cand win = best;
-        shfl_cand(win, found ? s + (ml & 0xFFu) : lane);
-        if (work && !found) {
-            if (n > P.max_leaf)
-                median = true;  // bvh/src/lib.rs:527-531
-            else
-                leaf = true;  // :576-579
+        // costs are positive, infinite or the default NaN: their bits order
+        // as total_cmp does, all below "none"
+        uint32_t best = kNoKey, win = 0;
+#pragma unroll
+        for (uint32_t a = 0; a < 3; ++a) {
+            float lb[6], gb[6];
+            uint32_t nl = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < 6; ++q) {
+                const uint32_t pre = (&T.pm[a][q][0])[static_cast<int>(cut[a]) - 1];
+                if (q == 0) nl = __popc(pre & node[0]);
+                lb[q] = __shfl_sync(kFull, R.val[q], top_bit(pre & node[q]));
+                gb[q] = __shfl_sync(kFull, R.val[q], top_bit(~pre & node[q]));
+            }
+            const uint32_t ng = n - nl;
+            if (ok[a] && cut[a] && nl >= P.min_leaf && ng >= P.min_leaf) {  // :407
+                const uint32_t ck = __float_as_uint(area.split_cost(surface_area6(lb), surface_area6(gb), nl, ng));
+                if (ck < best) {
+                    best = ck;
+                    win = (a << 8) | idx[a];
+                }
+            }
         }
-        if (found) {
-            axis = (ml >> 8) & 3u;
-            n_lt = win.n_lt;
-            if (n <= P.max_leaf && funkey(mh) >= leaf_cost(n)) leaf = true;  // :583
+        // first minimum of (cost, axis, index) in the segment: axis, and the
+        // lane that holds it
+        uint32_t axis, src;
+        if constexpr (kGeneral) {
+            win = (win << 8) | lane;  // one object per index: the lane breaks no tie
+            seg_min2(best, win, lane, ss, se, maxn);
+            axis = win >> 16;
+            src = win & 31u;
+        } else {
+            // indexes follow the lanes: the first lane of the lowest axis
+            const uint32_t own = best;
+            if (maxn == n0) {  // one segment
+                best = __reduce_min_sync(kFull, best);
+            } else {
+                for (uint32_t d = 1; d < maxn; d <<= 1) {
+                    const uint32_t u = __shfl_down_sync(kFull, best, d);
+                    if (lane + d < se) best = min(best, u);
+                }
+                best = __shfl_sync(kFull, best, ss);
+            }
+            const uint32_t w0 = __ballot_sync(kFull, own == best && win < 256u) & m,
+                           w1 = __ballot_sync(kFull, own == best && win < 512u) & m,
+                           w2 = __ballot_sync(kFull, own == best) & m;
+            axis = w0 ? 0u : (w1 ? 1u : 2u);
+            src = __ffs(w0 ? w0 : (w1 ? w1 : w2)) - 1;
         }
+        const bool found = live && best != kNoKey;
+        const uint32_t wcut =
+            (__shfl_sync(kFull, cut[0] | (cut[1] << 8) | (cut[2] << 16), src) >> (8u * axis)) & 63u;
+        const bool median = live && !found && n > P.max_leaf;  // bvh/src/lib.rs:527-531
+        const bool leaf = live && n <= P.max_leaf &&
+                          (!found || __uint_as_float(best) >= leaf_cost(n));  // :576-583
+        const bool split = found && !leaf;
+        // partition (bvh/src/lib.rs:597-612), stable
+        const bool pred = split && ((word >> (5u * axis)) & 31u) < wcut;
+        const uint32_t ltm = __ballot_sync(kFull, pred) & m;
+        uint32_t n_lt = __popc(ltm);
+        T.x[split ? (pred ? s + __popc(ltm & below) : s + n_lt + __popc(m & ~ltm & below)) : lane] = word;
+        __syncwarp();
+        word = T.x[lane];
+        __syncwarp();
+        if (split) {
+            const uint32_t side = lane < s + n_lt ? 0u : 0xFFFFFFFFu;
+#pragma unroll
+            for (uint32_t q = 0; q < kOrders; ++q) node[q] &= (&T.pm[axis][q][0])[static_cast<int>(wcut) - 1] ^ side;
+            if (n_lt == 0u || n_lt == n) {  // cannot happen: the winner has objects on both sides
+                set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
+                live = false;
+            }
+        }
+        bool odd = false;  // a median of other than two objects with equal centroids
         if (__any_sync(kFull, median)) {
             // median_split on axes 0, 1, 2 over the same list (:444-491, :528-530)
             const uint32_t half = n / 2u;
-            uint32_t best_ck = 0;
-            for (uint32_t a = 0; a < 3; ++a) {
-                const uint32_t key = fkey(center_of(sel3(lo, a), sel3(hi, a)));
-                uint32_t rank = 0;
-                for (uint32_t r = 0; r < maxn; ++r) {
-                    const bool use = median && r < n;
-                    const uint32_t kj = __shfl_sync(kFull, key, use ? s + r : lane);
-                    if (use) rank += (kj < key || (kj == key && s + r < lane)) ? 1u : 0u;
-                }
-                const bool pr = median && rank < half;
-                const uint32_t ltm = __ballot_sync(kFull, pr);
-                const uint32_t dst = median ? (pr ? s + __popc(ltm & m & below)
-                                                  : s + half + __popc(m & ~ltm & below))
-                                            : lane;
-                warp_exchange(dst, lane, lo, hi, id, xchg);
-                const bool in_lt = median && lane < s + half;
-                const bool in_gt = median && lane >= s + half;
-                float ml6[6], mg6[6];
+            bool same = true;  // two objects with equal centroids: the first is lt on every axis
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    ml6[i] = funkey(seg_min(in_lt ? fkey(lo[i]) : kKeyPosInf, lane, ss, se));
-                    mg6[i] = funkey(seg_min(in_gt ? fkey(lo[i]) : kKeyPosInf, lane, ss, se));
-                    ml6[3 + i] = funkey(seg_max(in_lt ? fkey(hi[i]) : kKeyNegInf, lane, ss, se));
-                    mg6[3 + i] = funkey(seg_max(in_gt ? fkey(hi[i]) : kKeyNegInf, lane, ss, se));
-                }
-                if (median) {
-                    const uint32_t ck =
-                        fkey(split_cost(surface_area6(ml6), surface_area6(mg6), sa_p, half, n - half));
-                    if (a == 0 || ck < best_ck) {
-                        best_ck = ck;
-                        axis = a;
-                        for (int i = 0; i < 6; ++i) {
-                            win.lt[i] = ml6[i];
-                            win.gt[i] = mg6[i];
-                        }
-                    }
+            for (int a = 0; a < 3; ++a) {
+                const uint32_t c = __float_as_uint(__shfl_sync(kFull, R.cen[a], (word >> (5 * a)) & 31u));
+                same &= c == __shfl_sync(kFull, c, lane == s ? s + 1u : s);
+            }
+            odd = median && !(n == 2u && same);
+            if (median) {
+                n_lt = half;
+                if (lane == s) n_median++;
+            }
+            if (__any_sync(kFull, odd)) {
+                MedianIo io;  // passed by address: copies, so that the loop's own stay in registers
+                io.word = word;
+                io.regs = R;
+#pragma unroll
+                for (int i = 0; i < 6; ++i) io.nb[i] = nb[i];
+                median_segments(odd, s, n, m, ss, se, maxn, T, io);
+                word = io.word;
+                if (odd) {
+#pragma unroll
+                    for (uint32_t q = 0; q < kOrders; ++q) node[q] = io.node[q];
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) nb[i] = io.nb[i];
                 }
             }
-            if (median) n_lt = half;
-            if (median && leader) n_median++;
-        }
-        // leaves of this level
-        if (live && leaf) {
-            if (leader) {
-                lane_store_node(O, nbase + slot, nb, base + s - tbase, n, 0u);
-                if (n > 1u) {
-                    n_holes++;
-                    if (depth == P.max_depth) n_capped++;
-                }
-            }
-            O.perm[base + lane] = id;
-        }
-        const bool split = work && !leaf;
-        // partition (bvh/src/lib.rs:597-612), stable; containment (:637-646)
+            if (median && !odd) {
+                const uint32_t bits = T.rt[word & 31u];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) c[a] = center_of(lo[a], hi[a]);
-        const float ca = axis == 0 ? c[0] : (axis == 1 ? c[1] : c[2]);
-        const bool pred = median ? lane < s + n_lt : ca < win.thr;
-        const uint32_t ltm = __ballot_sync(kFull, split && pred);
-        if (split && lane == s && static_cast<uint32_t>(__popc(ltm & m)) != n_lt)
-            set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
-        const bool ok = !split || box_contains2(win.lt, win.gt, pred, c[0], c[1], c[2]);
-        if (__any_sync(kFull, !ok) && lane == 0) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
-        if (split && leader) {
-            lane_store_node(O, nbase + slot, nb, base + s - tbase, n, pair);
-            any_split = true;
-            hmax = max(hmax, depth);
+                for (uint32_t q = 0; q < kOrders; ++q)
+                    node[q] = 1u << ((q < 6u ? bits >> (5u * q) : word >> (5u * (q - 6u))) & 31u);
+            }
         }
-        const uint32_t dst =
-            split ? (pred ? s + __popc(ltm & m & below) : s + n_lt + __popc(m & ~ltm & below)) : lane;
-        warp_exchange(dst, lane, lo, hi, id, xchg);
-        if (split) {
+        const bool parted = split || median;
+        float c[3];
+#pragma unroll
+        for (uint32_t a = 0; a < 3; ++a) c[a] = __shfl_sync(kFull, R.cen[a], (word >> (5u * a)) & 31u);
+#pragma unroll
+        for (uint32_t q = 0; q < 6; ++q) {
+            const float v = __shfl_sync(kFull, R.val[q], top_bit(node[q]));
+            if (parted && !odd) nb[q] = v;
+        }
+        if (parted) {
+            // containment of the centroids in their side's bounds (:637-646)
+            if (!box_contains(nb, c[0], c[1], c[2])) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
+            if (lane == s) hmax = max(hmax, depth + 1u);
             const uint32_t n_gt = n - n_lt;
             if (lane < s + n_lt) {
                 n = n_lt;
                 slot = pair + 1u;
                 pair = pair + 2u * n_gt;
-#pragma unroll
-                for (int i = 0; i < 6; ++i) nb[i] = win.lt[i];
             } else {
                 s = s + n_lt;
                 n = n_gt;
                 slot = pair;
                 pair = pair + 2u;
-#pragma unroll
-                for (int i = 0; i < 6; ++i) nb[i] = win.gt[i];
             }
             depth++;
-            // a child that the leaf rule stops (:556) is written now rather
-            // than by one more pass of the loop (the same node and entries)
-            if (n <= 1u || depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf)) {
-                if (lane == s) {
-                    lane_store_node(O, nbase + slot, nb, base + s - tbase, n, 0u);
-                    if (n > 1u) {
-                        n_holes++;
-                        if (depth == P.max_depth) n_capped++;
-                    }
+            // each child is written as it comes to be: a leaf where the leaf
+            // rule stops it (:556), else with its children's slots
+            const bool cleaf = leaf_rule(n, depth, P);
+            if (lane == s) {
+                lane_store_node(O, nbase + slot, nb, base + s - tbase, n, cleaf ? 0u : pair);
+                if (cleaf && n > 1u) {
+                    n_holes++;
+                    if (depth == P.max_depth) n_capped++;
                 }
-                O.perm[base + lane] = id;
+            }
+            if (cleaf) {
+                O.perm[base + lane] = T.ids[word & 31u];
                 live = false;
             }
         }
-        if (leaf) live = false;
+        if (leaf) {  // no split is worth it: the node was written as an inner one
+            if (lane == s) {
+                if (nbase + slot < O.node_cap) O.nodes[nbase + slot].child_node = 0u;
+                if (n > 1u) n_holes++;
+            }
+            O.perm[base + lane] = T.ids[word & 31u];
+            live = false;
+        }
     }
     // counters: one atomic per warp
-    const uint32_t hm = __reduce_max_sync(kFull, any_split ? hmax : 0u);
-    const bool anys = __any_sync(kFull, any_split);
+    const uint32_t hm = __reduce_max_sync(kFull, hmax);
     const uint32_t med = __reduce_add_sync(kFull, n_median);
     const uint32_t hol = __reduce_add_sync(kFull, n_holes);
     const uint32_t cap = __reduce_add_sync(kFull, n_capped);
     if (lane == 0) {
-        if (anys) atomicMax(&O.ctr->height, hm);
+        if (hm) atomicMax(&O.ctr->height, hm - 1u);
         if (med) atomicAdd(&O.ctr->median_splits, med);
         if (hol) atomicAdd(&O.ctr->holes, hol);
         if (cap) atomicAdd(&O.ctr->depth_capped, cap);

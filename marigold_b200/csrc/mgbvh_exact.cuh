@@ -55,14 +55,13 @@ __device__ __forceinline__ float center_of(float lo, float hi) {
 
 __device__ __forceinline__ float surface_area(float lx, float ly, float lz, float hx, float hy,
                                               float hz) {
-    if (hx < lx || hy < ly || hz < lz) return 0.0f;
     const float w = __fsub_rn(hx, lx);
     const float h = __fsub_rn(hy, ly);
     const float d = __fsub_rn(hz, lz);
     float s = __fmul_rn(w, h);
     s = __fadd_rn(s, __fmul_rn(w, d));
     s = __fadd_rn(s, __fmul_rn(h, d));
-    return __fmul_rn(2.0f, s);
+    return (hx < lx || hy < ly || hz < lz) ? 0.0f : __fmul_rn(2.0f, s);
 }
 
 __device__ __forceinline__ float surface_area6(const float* b) {
@@ -75,6 +74,46 @@ __device__ __forceinline__ float split_cost(float sa_lt, float sa_gt, float sa_p
     const float gt = __fmul_rn(__fmul_rn(__fdiv_rn(sa_gt, sa_p), kObjectCost), __uint2float_rn(n_gt));
     return __fadd_rn(__fadd_rn(kDepthCost, lt), gt);
 }
+
+// The parent's surface area as a divisor of many areas: the cost above, bit
+// for bit, with each quotient from the correctly rounded reciprocal
+// (P. W. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. R&D 34(1), 1990): one correction makes the
+// quotient faithful, a second one rounds it correctly, as long as no
+// intermediate leaves the normal range, which areas in [2^-60, 2^60] ensure
+// (the residuals are then multiples of at least 2^-149). Other areas divide.
+// The object cost multiplies the count instead of the quotient: both are
+// scalings by 8, so the rounded product is the same.
+struct NodeArea {
+    float area, rcp;
+    bool fast;
+
+    __device__ __forceinline__ explicit NodeArea(const float* box) {
+        area = surface_area6(box);
+        fast = area >= 8.673617379884035e-19f && area <= 1.152921504606847e18f;
+        rcp = __frcp_rn(fast ? area : 1.0f);
+    }
+
+    __device__ __forceinline__ float ratio(float x) const {
+        float q = __fmul_rn(x, rcp);
+        q = __fmaf_rn(__fmaf_rn(-area, q, x), rcp, q);
+        return __fmaf_rn(__fmaf_rn(-area, q, x), rcp, q);
+    }
+
+    __device__ __forceinline__ float split_cost(float sa_lt, float sa_gt, uint32_t n_lt, uint32_t n_gt) const {
+        float l, g;
+        if (fast && fminf(sa_lt, sa_gt) >= 8.673617379884035e-19f && fmaxf(sa_lt, sa_gt) <= 1.152921504606847e18f) {
+            l = ratio(sa_lt);
+            g = ratio(sa_gt);
+        } else {
+            l = __fdiv_rn(sa_lt, area);
+            g = __fdiv_rn(sa_gt, area);
+        }
+        l = __fmul_rn(l, __fmul_rn(kObjectCost, __uint2float_rn(n_lt)));
+        g = __fmul_rn(g, __fmul_rn(kObjectCost, __uint2float_rn(n_gt)));
+        return __fadd_rn(__fadd_rn(kDepthCost, l), g);
+    }
+};
 
 __device__ __forceinline__ float leaf_cost(uint32_t len) {  // bvh/src/lib.rs:251-253
     return __fmul_rn(kObjectCost, __uint2float_rn(len));
