@@ -56,6 +56,10 @@ constexpr int kTileThreads = 256;
 #endif
 constexpr int kMediumWarps = MGBVH_MEDIUM_WARPS;
 constexpr int kMediumThreads = kMediumWarps * 32;
+// Warps of the subtree CTA where there are too few subtrees to fill the SMs
+// with CTAs of kMediumWarps (medium_wide).
+constexpr int kWideWarps = 8;
+constexpr int kWidestWarps = 16;
 constexpr uint32_t kBinWords = 3 * 32 * 7;  // [axis][bin]{count, lo key xyz, hi key xyz}
 
 // Level counter slots rotate over three: level L reads ctr->lvl[L % 3],
@@ -1672,25 +1676,37 @@ struct MNodeExtra {
     uint32_t depth, ib;
 };
 
-// Shared memory of one subtree CTA for subtrees of up to kCap objects: the
-// records, two index lists, two node lists (every listed node holds more than
-// 32 objects and the nodes of one list are disjoint, so kCap / 33 + 1 entries
-// suffice) and per-warp bins.
-template <uint32_t kCap>
+// What the warps of a group share while they split one node together.
+template <int kWarps>
+struct MediumGroup {
+    uint32_t kind, axis, sbin, n_lt;  // kind: 0 split, 1 leaf, 2 partitioned already (median)
+    float thr;
+    uint32_t use_thr;      // the split is centroid < thr (learned form)
+    uint32_t wlt[kWarps];  // lt objects of each warp's slice
+    uint32_t keys[12];     // centroid keys of both sides
+    uint32_t bad;
+};
+
+// Shared memory of one subtree CTA of kWarps warps for subtrees of up to kCap
+// objects: the records (rhi.w holds an object's bin codes), two index lists,
+// two node lists (every listed node holds more than 32 objects and the nodes
+// of one list are disjoint, so kCap / 33 + 1 entries suffice) and per-warp
+// bins.
+template <uint32_t kCap, int kWarps>
 struct MediumSmemT {
     static constexpr uint32_t kListCap = kCap / (kSmallMax + 1) + 1;
+    static constexpr int kW = kWarps;
     float4 rlo[kCap];
     float4 rhi[kCap];
     uint16_t idx[2][kCap];
     MNode list[2][kListCap];
     MNodeExtra list_x[2][kListCap];
-    uint32_t bins[kMediumWarps][kBinWords];
+    uint32_t bins[kWarps][kSweepWords];
+    MediumGroup<kWarps> grp[kWarps > 1 ? kWarps / 2 : 1];
     uint32_t list_n[2];
-    uint32_t rootk[12];
+    uint32_t rootk[6];
 };
-using MediumSmem = MediumSmemT<kMediumMax>;
 constexpr uint32_t kMediumSmallCap = 512;  // the instance for medium_max <= 512 (more CTAs per SM)
-using MediumSmemSmall = MediumSmemT<kMediumSmallCap>;
 
 // A subtree of <= 32 objects split off inside a subtree CTA of the persistent
 // build: its objects are idx[ob][cs .. cs + len) of the CTA's records, built
@@ -1708,30 +1724,24 @@ struct SmallRef {
 // kCap / 2: disjoint subtrees of at least 2 objects) and each warp's tables
 // to build them.
 template <uint32_t kCap>
-struct MediumSmemQ : MediumSmemT<kCap> {
+struct MediumSmemQ : MediumSmemT<kCap, kMediumWarps> {
     SubtreeSmem tables[kMediumWarps];
     SmallRef sref[kCap / 2];
     uint32_t sref_n;
 };
 
-template <class MS>
-__device__ __forceinline__ void medium_load_warp_records(const MS& S, uint32_t ib, uint32_t s,
-                                                         uint32_t n, uint32_t lane, float* lo,
-                                                         float* hi, uint32_t& id) {
-    if (lane < n) {
-        const uint32_t r = S.idx[ib][s + lane];
-        const float4 a = S.rlo[r], b = S.rhi[r];
-        lo[0] = a.x;
-        lo[1] = a.y;
-        lo[2] = a.z;
-        id = __float_as_uint(a.w);
-        hi[0] = b.x;
-        hi[1] = b.y;
-        hi[2] = b.z;
-    } else {
-        lo[0] = lo[1] = lo[2] = hi[0] = hi[1] = hi[2] = 0.0f;
-        id = 0;
+// Barrier among the `warps` warps of group g of at most kGroups (barrier 0 is
+// the CTA's). Constant barrier numbers: with a run-time one the CTA would be
+// given all 16, and fewer CTAs fit an SM.
+template <int kGroups>
+__device__ __forceinline__ void group_sync(uint32_t g, uint32_t warps) {
+    if constexpr (kGroups > 1) {
+        if (g + 1u < kGroups) {
+            group_sync<kGroups - 1>(g, warps);
+            return;
+        }
     }
+    asm volatile("bar.sync %0, %1;" ::"n"(kGroups), "r"(warps * 32u) : "memory");
 }
 
 // Warp: finish a leaf of the medium subtree (record + permutation).
@@ -1749,21 +1759,38 @@ __device__ __forceinline__ void medium_leaf(const MS& S, uint32_t ib, uint32_t b
     }
 }
 
-// Warp: stable partition of [s, s+n) from idx[ib] into idx[ib^1] by pred(p);
-// returns the lt count; accumulates child centroid keys.
-// With clt non-null, also checks each centroid against its side's child box
-// (clt for lt, cgt for gt) and sets bad where one lies outside.
+// Centroid bounds of the lt and gt objects a lane has placed, and whether one
+// of them was NaN (which no bounds contain).
+struct SideBounds {
+    float lt[6], gt[6];  // min xyz, max xyz
+    bool nan;
+
+    __device__ __forceinline__ SideBounds() : nan(false) {
+        box_empty(lt);
+        box_empty(gt);
+    }
+    __device__ __forceinline__ void add(bool first, const float* c) {
+        nan |= c[0] != c[0] || c[1] != c[1] || c[2] != c[2];
+        if (first)
+            box_grow(lt, c[0], c[1], c[2], c[0], c[1], c[2]);
+        else
+            box_grow(gt, c[0], c[1], c[2], c[0], c[1], c[2]);
+    }
+};
+
+// Warp: stable partition of positions [p0, p1) of a node's list idx[ib] into
+// idx[ib ^ 1]: lt objects from position `lt_at` on, gt objects from `gt_at`
+// on, both within [s, s + n). Returns the lt count; `side` takes the centroids.
+// pred(p, r, c): position, record, centroid.
 template <class MS, class Pred>
-__device__ __forceinline__ uint32_t medium_partition(MS& S, uint32_t ib, uint32_t s,
-                                                     uint32_t n, uint32_t n_lt_expect, uint32_t lane,
-                                                     Pred pred, uint32_t* k /*12*/,
-                                                     const float* clt = nullptr,
-                                                     const float* cgt = nullptr, bool* bad = nullptr) {
+__device__ __forceinline__ uint32_t medium_partition(MS& S, uint32_t ib, uint32_t s, uint32_t n, uint32_t p0,
+                                                     uint32_t p1, uint32_t lt_at, uint32_t gt_at, uint32_t lane,
+                                                     Pred pred, SideBounds& side) {
     const uint32_t below = (1u << lane) - 1u;
-    uint32_t lt_run = 0, gt_run = 0;
-    for (uint32_t b0 = s; b0 < s + n; b0 += 32) {
+    const uint32_t lt0 = lt_at;
+    for (uint32_t b0 = p0; b0 < p1; b0 += 32) {
         const uint32_t p = b0 + lane;
-        const bool valid = p < s + n;
+        const bool valid = p < p1;
         uint32_t r = 0;
         float c[3] = {0.f, 0.f, 0.f};
         bool pr = false;
@@ -1773,28 +1800,20 @@ __device__ __forceinline__ uint32_t medium_partition(MS& S, uint32_t ib, uint32_
             c[0] = center_of(a.x, b.x);
             c[1] = center_of(a.y, b.y);
             c[2] = center_of(a.z, b.z);
-            pr = pred(p, c);
+            pr = pred(p, __float_as_uint(b.w), c);
         }
         const uint32_t m = __ballot_sync(kFull, pr);
         const uint32_t vm = __ballot_sync(kFull, valid);
         if (valid) {
-            const uint32_t dst = pr ? s + lt_run + __popc(m & below)
-                                    : s + n_lt_expect + gt_run + __popc(vm & ~m & below);
-            if (dst < s + n) S.idx[ib ^ 1u][dst] = static_cast<uint16_t>(r);
-            grow_keys12(k, pr, c);
-            if (clt) *bad |= !box_contains2(clt, cgt, pr, c[0], c[1], c[2]);
+            const uint32_t dst = pr ? lt_at + __popc(m & below) : gt_at + __popc(vm & ~m & below);
+            if (dst - s < n) S.idx[ib ^ 1u][dst] = static_cast<uint16_t>(r);
+            side.add(pr, c);
         }
-        lt_run += __popc(m);
-        gt_run += __popc(vm & ~m);
+        lt_at += __popc(m);
+        gt_at += __popc(vm & ~m);
     }
     __syncwarp();
-    return lt_run;
-}
-
-__device__ __forceinline__ void warp_reduce_keys12(uint32_t* k) {
-#pragma unroll
-    for (int q = 0; q < 12; ++q)
-        k[q] = ((q % 6) < 3) ? __reduce_min_sync(kFull, k[q]) : __reduce_max_sync(kFull, k[q]);
+    return lt_at - lt0;
 }
 
 // The learned form at one binned node of the medium phase (warp-uniform):
@@ -1816,12 +1835,11 @@ template <class MS>
 __device__ MGBVH_LEARNED_NODE_ATTR void learned_node(const MS& S, const Learn& LN, const Params& P,
                                           const MNode& nd, uint32_t ib, uint32_t base, uint32_t s,
                                           uint32_t n, uint32_t depth, uint32_t tbase,
-                                          const uint32_t* cnt, const float* ext,
-                                          uint32_t plain_ck, uint32_t lane, Cand& win,
-                                          uint32_t& axis, uint32_t& n_lt, bool& use_thr,
-                                          uint32_t* wb) {
+                                          const float* ext, uint32_t lane, SweepResult& w,
+                                          float& out_thr, bool& use_thr, uint32_t* wb) {
+    const uint32_t plain_ck = w.cost | 0x80000000u;  // fkey of a cost (never negative)
     float f[24];
-    node_features(nd.b, nd.cb, n, depth, cnt, f);
+    node_features(nd.b, nd.cb, n, depth, w.cnt, f);
     const float sa_p = surface_area6(nd.b);
     auto fetch = [&](uint32_t j, float* lo, float* hi) {
         const uint32_t r = S.idx[ib][s + j];
@@ -1928,14 +1946,14 @@ __device__ MGBVH_LEARNED_NODE_ATTR void learned_node(const MS& S, const Learn& L
                         }
                     }
                     if (!valid) continue;
-                    uint32_t* w = wb + (q * 17 + a) * 7;
-                    atomicAdd(w, 1u);
-                    atomicMin(w + 1, fkey(lo[0]));
-                    atomicMin(w + 2, fkey(lo[1]));
-                    atomicMin(w + 3, fkey(lo[2]));
-                    atomicMax(w + 4, fkey(hi[0]));
-                    atomicMax(w + 5, fkey(hi[1]));
-                    atomicMax(w + 6, fkey(hi[2]));
+                    uint32_t* w7 = wb + (q * 17 + a) * 7;
+                    atomicAdd(w7, 1u);
+                    atomicMin(w7 + 1, fkey(lo[0]));
+                    atomicMin(w7 + 2, fkey(lo[1]));
+                    atomicMin(w7 + 3, fkey(lo[2]));
+                    atomicMax(w7 + 4, fkey(hi[0]));
+                    atomicMax(w7 + 5, fkey(hi[1]));
+                    atomicMax(w7 + 6, fkey(hi[2]));
                 }
             }
             __syncwarp();
@@ -1972,9 +1990,14 @@ __device__ MGBVH_LEARNED_NODE_ATTR void learned_node(const MS& S, const Learn& L
             const uint32_t wlo = static_cast<uint32_t>(wk2);
             if (wlo != kNoKey && static_cast<uint32_t>(wk2 >> 32) < plain_ck) {
                 shfl_cand(c, wlo & 0xFFu);
-                win = c;
-                axis = (wlo >> 8) & 3u;
-                n_lt = c.n_lt;
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    w.lt[i] = c.lt[i];
+                    w.gt[i] = c.gt[i];
+                }
+                w.axis = (wlo >> 8) & 3u;
+                w.n_lt = c.n_lt;
+                out_thr = c.thr;
                 use_thr = true;
             }
         }
@@ -1990,7 +2013,70 @@ __global__ void transpose_weights_kernel(const __nv_bfloat16* __restrict__ w, __
     t[i] = src >= 0 ? w[src] : __float2bfloat16_rn(0.0f);
 }
 
-// One CTA builds the subtree of one medium node (33..1024 objects).
+// median_split on axes 0, 1, 2 over the same list (bvh/src/lib.rs:444-491,
+// 528-530) by one warp: stable selection of the n/2 smallest centroid keys. The
+// list ends in idx[ib ^ 1]; w takes the cheapest axis's boxes and the lt count,
+// side the final halves' centroids.
+template <class MS>
+__device__ __forceinline__ void median_node(MS& S, const MNode& nd, uint32_t ib, uint32_t s, uint32_t n, uint32_t lane,
+                                         SweepResult& w, SideBounds& side) {
+    const uint32_t half = n / 2u;
+    uint32_t cb = ib, best_ck = 0;
+    for (uint32_t a = 0; a < 3; ++a) {
+        side = SideBounds();
+        medium_partition(
+            S, cb, s, n, s, s + n, s, s + half, lane,
+            [&](uint32_t p, uint32_t, const float* c) {
+                const uint32_t key = fkey(sel3(c, a));
+                uint32_t rank = 0;
+                for (uint32_t q = s; q < s + n; ++q) {
+                    const uint32_t r = S.idx[cb][q];
+                    const uint32_t kq = fkey(center_of(a == 0 ? S.rlo[r].x : (a == 1 ? S.rlo[r].y : S.rlo[r].z),
+                                                       a == 0 ? S.rhi[r].x : (a == 1 ? S.rhi[r].y : S.rhi[r].z)));
+                    rank += (kq < key || (kq == key && q < p)) ? 1u : 0u;
+                }
+                return rank < half;
+            },
+            side);
+        cb ^= 1u;
+        float blt[6], bgt[6];
+        box_empty(blt);
+        box_empty(bgt);
+        for (uint32_t p = s + lane; p < s + n; p += 32) {
+            const uint32_t r = S.idx[cb][p];
+            const float4 lo = S.rlo[r], hi = S.rhi[r];
+            box_grow2(blt, bgt, p < s + half, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            blt[i] = i < 3 ? warp_min(blt[i]) : warp_max(blt[i]);
+            bgt[i] = i < 3 ? warp_min(bgt[i]) : warp_max(bgt[i]);
+        }
+        const uint32_t key =
+            fkey(split_cost(surface_area6(blt), surface_area6(bgt), surface_area6(nd.b), half, n - half));
+        if (a == 0 || key < best_ck) {
+            best_ck = key;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                w.lt[i] = blt[i];
+                w.gt[i] = bgt[i];
+            }
+        }
+    }
+    w.n_lt = half;
+}
+
+// A node of the subtree as the warps that split it see it.
+struct MSplit {
+    uint32_t s, n, depth, ib;
+    BinMap map[3];
+};
+
+// One CTA builds the subtree of one medium node (33..kCap objects). The nodes
+// of one depth are split together, a warp each; where a depth has at most half
+// as many nodes as the CTA has warps, groups of warps split a node together
+// (they bin and partition slices of it; the group's first warp sweeps the bins
+// and emits the children).
 // kQueue (the persistent batched build): records are read through L2 only,
 // and each subtree of <= 32 objects is built at once by the warp that split
 // it off, from shared memory, instead of going to the small list.
@@ -1998,31 +2084,32 @@ template <bool kLearn, class MS, bool kQueue = false, bool kGeneral = false>
 __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec* rec1,
                                             Task* small, uint32_t cap_small, const Params& P,
                                             const Out& O, const Learn& LN) {
+    constexpr uint32_t kW = MS::kW;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     Rec* src = (t.buf ? rec1 : rec0) + t.start;
     const uint32_t base = t.start;
-    uint32_t k[12];
-    init_key12(k);
-    if (threadIdx.x < 12) S.rootk[threadIdx.x] = ((threadIdx.x % 6) < 3) ? kKeyPosInf : kKeyNegInf;
+    if (threadIdx.x < 6) S.rootk[threadIdx.x] = threadIdx.x < 3 ? kKeyPosInf : kKeyNegInf;
     if (threadIdx.x < 2) S.list_n[threadIdx.x] = 0;
     if constexpr (kQueue) {
         if (threadIdx.x == 0) S.sref_n = 0;
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < t.len; i += blockDim.x) {
+    float cb[6];
+    box_empty(cb);
+    for (uint32_t i = threadIdx.x; i < t.len; i += kW * 32u) {
         const Rec r = load_rec<kQueue>(src + i);
         S.rlo[i] = r.lo;
         S.rhi[i] = r.hi;
         S.idx[0][i] = static_cast<uint16_t>(i);
-        accum_keys(k, r.lo.x, r.lo.y, r.lo.z, r.hi.x, r.hi.y, r.hi.z);
+        const float c[3] = {center_of(r.lo.x, r.hi.x), center_of(r.lo.y, r.hi.y), center_of(r.lo.z, r.hi.z)};
+        box_grow(cb, c[0], c[1], c[2], c[0], c[1], c[2]);
     }
-    // root centroid bounds (keys 6..11)
+    // root centroid bounds
 #pragma unroll
-    for (int q = 6; q < 12; ++q) {
-        const bool is_min = q < 9;
-        const uint32_t v = is_min ? __reduce_min_sync(kFull, k[q]) : __reduce_max_sync(kFull, k[q]);
+    for (int q = 0; q < 6; ++q) {
+        const uint32_t v = q < 3 ? __reduce_min_sync(kFull, fkey(cb[q])) : __reduce_max_sync(kFull, fkey(cb[q]));
         if (lane == 0) {
-            if (is_min)
+            if (q < 3)
                 atomicMin(&S.rootk[q], v);
             else
                 atomicMax(&S.rootk[q], v);
@@ -2034,8 +2121,8 @@ __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec*
         for (int a = 0; a < 3; ++a) {
             r.b[a] = t.lo[a];
             r.b[3 + a] = t.hi[a];
-            r.cb[a] = funkey(S.rootk[6 + a]);
-            r.cb[3 + a] = funkey(S.rootk[9 + a]);
+            r.cb[a] = funkey(S.rootk[a]);
+            r.cb[3 + a] = funkey(S.rootk[3 + a]);
         }
         r.s = 0;
         r.n = t.len;
@@ -2045,276 +2132,286 @@ __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec*
         S.list_x[0][0].ib = 0;
         S.list_n[0] = 1;
     }
+    const uint32_t B = P.bins ? P.bins : 32u;
     uint32_t cur = 0;
-    uint32_t hmax = 0;
-    bool any_split = false;
+    uint32_t hmax = 0;  // depth + 1 of the deepest split
     uint32_t n_median = 0;
+
+    // One warp: writes the node and its children. ck: both sides' centroid
+    // bounds (lt min xyz, lt max xyz, gt min xyz, gt max xyz).
+    auto emit = [&](const MNode& nd, const MSplit& m, const float* lt, const float* gt, uint32_t n_lt,
+                    const float* ck, bool bad) {
+        const uint32_t s = m.s, n = m.n, ob = m.ib ^ 1u;
+        // every centroid of a side inside its box (bvh/src/lib.rs:637-646):
+        // the corners of the side's centroid bounds
+        bad |= !box_contains(lt, ck[0], ck[1], ck[2]) || !box_contains(lt, ck[3], ck[4], ck[5]) ||
+               !box_contains(gt, ck[6], ck[7], ck[8]) || !box_contains(gt, ck[9], ck[10], ck[11]);
+        if (bad && lane == 0) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
+        warp_store_node(O, t.nbase + nd.slot, nd.b, base + s - t.tbase, n, nd.pair, lane);
+        hmax = max(hmax, m.depth + 1u);
+        const uint32_t n_gt = n - n_lt, cdepth = m.depth + 1u;
+        // each child's class (0 leaf, 1 another node of this CTA, 2 a subtree
+        // of <= 32 objects), then one atomic per list for both children: lane 0
+        // the CTA's list, lane 1 the small list
+        uint32_t cls[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t len = c == 0 ? n_gt : n_lt;
+            cls[c] = leaf_rule(len, cdepth, P) ? 0u : (len > kSmallMax ? 1u : 2u);
+        }
+        uint32_t at = 0;
+        const uint32_t nn = (cls[0] == 1u) + (cls[1] == 1u), ns = (cls[0] == 2u) + (cls[1] == 2u);
+        if (lane == 0 && nn) at = atomicAdd(&S.list_n[cur ^ 1u], nn);
+        if (lane == 1 && ns) {
+            if constexpr (kQueue)
+                at = atomicAdd(&S.sref_n, ns);
+            else
+                at = atomicAdd(&O.ctr->n_small, ns);
+        }
+        const uint32_t at_node = __shfl_sync(kFull, at, 0), at_small = __shfl_sync(kFull, at, 1);
+#pragma unroll  // constant c: the child's box and bounds stay in registers
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t len = c == 0 ? n_gt : n_lt;
+            const uint32_t cs = c == 0 ? s + n_lt : s;
+            const uint32_t slot = c == 0 ? nd.pair : nd.pair + 1u;
+            const uint32_t pair = c == 0 ? nd.pair + 2u : nd.pair + 2u * n_gt;
+            const float* cbx = c == 0 ? gt : lt;
+            const float* cck = c == 0 ? ck + 6 : ck;
+            // after the gt child where both go to the same list
+            const uint32_t second = c == 1 && cls[0] == cls[1] ? 1u : 0u;
+            if (cls[c] == 0u) {
+                medium_leaf(S, ob, base, cs, len, slot, cdepth, cbx, t.nbase, t.tbase, P, O, lane);
+            } else if (cls[c] == 1u) {
+                if (lane == 0) {
+                    MNode q;
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        q.b[i] = cbx[i];
+                        q.cb[i] = cck[i];
+                    }
+                    q.s = cs;
+                    q.n = len;
+                    q.slot = slot;
+                    q.pair = pair;
+                    S.list[cur ^ 1u][at_node + second] = q;
+                    S.list_x[cur ^ 1u][at_node + second].depth = cdepth;
+                    S.list_x[cur ^ 1u][at_node + second].ib = ob;
+                }
+            } else {
+                if constexpr (kQueue) {
+                    // the persistent build: listed, and built from shared memory
+                    // once the CTA's own nodes are done
+                    if (lane == 0) {
+                        SmallRef& q = S.sref[at_small + second];
+                        for (int i = 0; i < 6; ++i) q.b[i] = cbx[i];
+                        q.slot = slot;
+                        q.pair = pair;
+                        q.depth = cdepth;
+                        q.cs = static_cast<uint16_t>(cs);
+                        q.len = static_cast<uint8_t>(len);
+                        q.ob = static_cast<uint8_t>(ob);
+                    }
+                    continue;
+                }
+                // subtree of <= 32 objects: write its records back to this task's
+                // range of the record buffer and queue it for small_kernel
+                if (lane < len) {
+                    const uint32_t r = S.idx[ob][cs + lane];
+                    Rec rr;
+                    rr.lo = S.rlo[r];
+                    rr.hi = S.rhi[r];
+                    src[cs + lane] = rr;
+                }
+                const uint32_t si = at_small + second;
+                if (si >= cap_small) {
+                    if (lane == 0) set_error(O.ctr, MGBVH_ERR_CAPACITY, kSiteCapacity);
+                } else if (lane == 0) {
+                    Task st;
+                    for (int a = 0; a < 3; ++a) {
+                        st.lo[a] = cbx[a];
+                        st.hi[a] = cbx[3 + a];
+                    }
+                    st.start = base + cs;
+                    st.len = len;
+                    st.slot = slot;
+                    st.pair = pair;
+                    st.depth = cdepth;
+                    st.buf = t.buf;
+                    st.tile0 = st.ntiles = 0;
+                    st.nbase = t.nbase;
+                    st.tbase = t.tbase;
+                    small[si] = st;
+                }
+            }
+        }
+    };
+
     for (;;) {
         __syncthreads();
         const uint32_t ncur = S.list_n[cur];
         if (ncur == 0) break;
         if (threadIdx.x == 0) S.list_n[cur ^ 1u] = 0;
         __syncthreads();
-        for (uint32_t li = warp; li < ncur; li += kMediumWarps) {
+        // warps per node: 1, or the largest power of two that the depth's
+        // nodes leave
+        uint32_t G = 1;
+        while (2u * G * ncur <= kW) G <<= 1;
+        for (uint32_t li = warp / G; li < ncur; li += kW / G) {
+            const uint32_t g = warp / G, gw = warp % G, gt = gw * 32u + lane;
+            MediumGroup<static_cast<int>(kW)>& D = S.grp[G > 1u ? g : 0u];
+            auto sync = [&]() {
+                if (G > 1u)
+                    group_sync<static_cast<int>(kW) / 2>(g, G);
+                else
+                    __syncwarp();
+            };
             const MNode nd = S.list[cur][li];
-            const MNodeExtra nx = S.list_x[cur][li];
-            const uint32_t s = nd.s, n = nd.n, depth = nx.depth, ib = nx.ib;
-            bool leaf = depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf);
-            Cand win;
-            uint32_t axis = 0, sbin = 0, n_lt = 0;
-            bool median = false;
-            bool use_thr = false;  // the learned form replaced the binned split
-            const uint32_t B = P.bins ? P.bins : 32u;
-            float ext[3];
-            bool axis_ok[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                ext[a] = __fsub_rn(nd.cb[3 + a], nd.cb[a]);
-                axis_ok[a] = !(ext[a] == 0.0f);
-            }
-            if (!leaf) {
-                uint32_t* wb = S.bins[warp];
-                init_task_bins(wb, lane, 32);
-                __syncwarp();
-                for (uint32_t p = s + lane; p < s + n; p += 32) {
-                    const uint32_t r = S.idx[ib][p];
-                    const float4 lo = S.rlo[r], hi = S.rhi[r];
-                    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        if (!axis_ok[a]) continue;
-                        const uint32_t b = bin_of(center_of(l[a], h[a]), nd.cb[a], ext[a], B);
-                        uint32_t* bw = wb + (a * 32 + b) * 7;
-                        atomicAdd(bw, 1u);
-                        atomicMin(bw + 1, fkey(l[0]));
-                        atomicMin(bw + 2, fkey(l[1]));
-                        atomicMin(bw + 3, fkey(l[2]));
-                        atomicMax(bw + 4, fkey(h[0]));
-                        atomicMax(bw + 5, fkey(h[1]));
-                        atomicMax(bw + 6, fkey(h[2]));
-                    }
-                }
-                __syncwarp();
-                uint32_t cnt[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) cnt[a] = wb[(a * 32 + lane) * 7];
-                // each axis's bin read from the warp's bins as the sweep
-                // reaches it (fewer live registers)
-                Cand best;
-                binned_candidates_f(
-                    [&](uint32_t a, uint32_t& ca, float* ba) {
-                        const uint32_t* bw = wb + (a * 32 + lane) * 7;
-                        ca = bw[0];
-#pragma unroll
-                        for (int i = 0; i < 6; ++i) ba[i] = funkey(bw[1 + i]);
-                    },
-                    axis_ok, B, n, surface_area6(nd.b), P, lane, best);
-                const uint64_t wk = warp_min_key(best.key);
-                const uint32_t wlo = static_cast<uint32_t>(wk);
-                if (wlo == kNoKey) {
-                    if (n > P.max_leaf)
-                        median = true;
-                    else
-                        leaf = true;
-                } else {
-                    axis = (wlo >> 8) & 3u;
-                    sbin = wlo & 0xFFu;
-                    win = best;
-                    shfl_cand(win, sbin);
-                    const float cost = funkey(static_cast<uint32_t>(wk >> 32));
-                    if (n <= P.max_leaf && cost >= leaf_cost(n)) leaf = true;
-                    n_lt = win.n_lt;
-                    if constexpr (kLearn) {
-                        if (!leaf && (LN.w || LN.samples) && B == 32u)
-                            learned_node(S, LN, P, nd, ib, base, s, n, depth, t.tbase, cnt, ext,
-                                         static_cast<uint32_t>(wk >> 32), lane, win, axis, n_lt,
-                                         use_thr, S.bins[warp]);
-                        if (use_thr && lane == 0) atomicAdd(&O.ctr->learned, 1u);
-                    }
-                }
-            }
-            if (leaf) {
-                medium_leaf(S, ib, base, s, n, nd.slot, depth, nd.b, t.nbase, t.tbase, P, O, lane);
-                continue;
-            }
-            uint32_t ck[12];
-            init_key12(ck);
-            uint32_t ob = ib ^ 1u;
-            // containment of centroids in child bounds (bvh/src/lib.rs:637-646),
-            // checked on the pass that places each object
+            MSplit m;
+            m.s = nd.s;
+            m.n = nd.n;
+            m.depth = S.list_x[cur][li].depth;
+            m.ib = S.list_x[cur][li].ib;
+            uint32_t kind = 1;
+            SweepResult w;
+            float ck[12];
             bool bad = false;
-            if (!median) {
-                const float cmin = sel3(nd.cb, axis), ex = sel3(ext, axis), thr = win.thr;
-                const bool by_thr = use_thr;
-                const uint32_t got = medium_partition(
-                    S, ib, s, n, n_lt, lane,
-                    [&](uint32_t, const float* c) {
-                        const float ca = sel3(c, axis);
-                        return by_thr ? ca < thr : bin_of(ca, cmin, ex, B) < sbin;
-                    },
-                    ck, win.lt, win.gt, &bad);
-                if (got != n_lt && lane == 0) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
-            } else {
-                // median_split on axes 0, 1, 2 over the same list (bvh/src/lib.rs:444-491,
-                // 528-530): stable selection of the n/2 smallest centroid keys.
-                const uint32_t m = n / 2u;
-                uint32_t cb = ib;
-                uint32_t best_ck = 0;
-                for (uint32_t a = 0; a < 3; ++a) {
-                    uint32_t dummy[12];
-                    init_key12(dummy);
-                    medium_partition(
-                        S, cb, s, n, m, lane,
-                        [&](uint32_t p, const float* c) {
-                            const uint32_t key = fkey(sel3(c, a));
-                            uint32_t rank = 0;
-                            for (uint32_t q = s; q < s + n; ++q) {
-                                const uint32_t r = S.idx[cb][q];
-                                const uint32_t kq = fkey(center_of(
-                                    a == 0 ? S.rlo[r].x : (a == 1 ? S.rlo[r].y : S.rlo[r].z),
-                                    a == 0 ? S.rhi[r].x : (a == 1 ? S.rhi[r].y : S.rhi[r].z)));
-                                rank += (kq < key || (kq == key && q < p)) ? 1u : 0u;
+            if (!leaf_rule(m.n, m.depth, P)) {
+                uint32_t* wb = S.bins[warp - gw];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) m.map[a] = BinMap(nd.cb[a], nd.cb[3 + a], B);
+                clear_bins(wb, gt, G * 32u);
+                sync();
+                for (uint32_t p = m.s + gt; p < m.s + m.n; p += G * 32u) {
+                    const uint32_t r = S.idx[m.ib][p];
+                    const float4 hi = S.rhi[r];
+                    S.rhi[r].w = __uint_as_float(add_to_bins(wb, m.map, S.rlo[r], hi));
+                }
+                if (G > 1u && gt < 12u) D.keys[gt] = (gt % 6u) < 3u ? kKeyPosInf : kKeyNegInf;
+                sync();
+                float thr = 0.0f;
+                bool use_thr = false;
+                SideBounds side;
+                if (gw == 0u) {
+                    w = sweep_bins(wb, m.map, m.n, NodeArea(nd.b), P, lane);
+                    if (!w.found)
+                        kind = m.n > P.max_leaf ? 2u : 1u;
+                    else
+                        kind = m.n <= P.max_leaf && __uint_as_float(w.cost) >= leaf_cost(m.n) ? 1u : 0u;
+                    if constexpr (kLearn) {
+                        if (kind == 0u && (LN.w || LN.samples) && B == 32u) {
+                            const float ext[3] = {m.map[0].ext, m.map[1].ext, m.map[2].ext};
+                            learned_node(S, LN, P, nd, m.ib, base, m.s, m.n, m.depth, t.tbase, ext, lane, w, thr,
+                                         use_thr, wb);
+                            if (use_thr && lane == 0) atomicAdd(&O.ctr->learned, 1u);
+                        }
+                    }
+                    if (kind == 2u) {
+                        median_node(S, nd, m.ib, m.s, m.n, lane, w, side);
+                        n_median++;
+                    }
+                    if (G > 1u && lane == 0) {
+                        D.kind = kind;
+                        D.axis = w.axis;
+                        D.sbin = w.bin;
+                        D.n_lt = w.n_lt;
+                        D.thr = thr;
+                        D.use_thr = use_thr ? 1u : 0u;
+                        D.bad = 0u;
+                    }
+                }
+                if (G > 1u) {
+                    sync();
+                    if (gw) {
+                        kind = D.kind;
+                        w.axis = D.axis;
+                        w.bin = D.sbin;
+                        w.n_lt = D.n_lt;
+                        thr = D.thr;
+                        use_thr = D.use_thr != 0u;
+                    }
+                }
+                if (kind == 0u) {
+                    // each warp places a slice of whole 32s; in a group, the
+                    // slices' lt counts come first
+                    const uint32_t sh = 5u * w.axis, sbin = w.bin, axis = w.axis;
+                    const uint32_t per = ((m.n + G * 32u - 1u) / (G * 32u)) * 32u;
+                    const uint32_t p0 = m.s + min(gw * per, m.n), p1 = m.s + min((gw + 1u) * per, m.n);
+                    auto pred = [&](uint32_t, uint32_t code, const float* c) {
+                        return kLearn && use_thr ? sel3(c, axis) < thr : ((code >> sh) & 31u) < sbin;
+                    };
+                    uint32_t lt_at = 0;
+                    if (G > 1u) {
+                        uint32_t cnt = 0;
+                        for (uint32_t b0 = p0; b0 < p1; b0 += 32) {
+                            const uint32_t p = b0 + lane;
+                            bool pr = false;
+                            if (p < p1) {
+                                const uint32_t r = S.idx[m.ib][p];
+                                const float4 hi = S.rhi[r];
+                                float c[3] = {0.f, 0.f, 0.f};
+                                if (kLearn && use_thr) {
+                                    const float4 lo = S.rlo[r];
+                                    c[0] = center_of(lo.x, hi.x);
+                                    c[1] = center_of(lo.y, hi.y);
+                                    c[2] = center_of(lo.z, hi.z);
+                                }
+                                pr = pred(p, __float_as_uint(hi.w), c);
                             }
-                            return rank < m;
-                        },
-                        dummy);
-                    cb ^= 1u;
-                    float blt[6], bgt[6];
-                    box_empty(blt);
-                    box_empty(bgt);
-                    for (uint32_t p = s + lane; p < s + n; p += 32) {
-                        const uint32_t r = S.idx[cb][p];
-                        const float4 lo = S.rlo[r], hi = S.rhi[r];
-                        box_grow2(blt, bgt, p < s + m, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
-                    }
-                    for (int i = 0; i < 3; ++i) {
-                        blt[i] = funkey(__reduce_min_sync(kFull, fkey(blt[i])));
-                        bgt[i] = funkey(__reduce_min_sync(kFull, fkey(bgt[i])));
-                        blt[3 + i] = funkey(__reduce_max_sync(kFull, fkey(blt[3 + i])));
-                        bgt[3 + i] = funkey(__reduce_max_sync(kFull, fkey(bgt[3 + i])));
-                    }
-                    const float cost = split_cost(surface_area6(blt), surface_area6(bgt),
-                                                  surface_area6(nd.b), m, n - m);
-                    const uint32_t key = fkey(cost);
-                    if (a == 0 || key < best_ck) {
-                        best_ck = key;
-                        for (int i = 0; i < 6; ++i) {
-                            win.lt[i] = blt[i];
-                            win.gt[i] = bgt[i];
+                            cnt += __popc(__ballot_sync(kFull, pr));
                         }
+                        if (lane == 0) D.wlt[gw] = cnt;
+                        sync();
+                        for (uint32_t q = 0; q < gw; ++q) lt_at += D.wlt[q];
                     }
+                    const uint32_t got = medium_partition(S, m.ib, m.s, m.n, p0, p1, m.s + lt_at,
+                                                          m.s + w.n_lt + (p0 - m.s - lt_at), lane, pred, side);
+                    // (the last slice's count completes the node's)
+                    if (gw == G - 1u && lt_at + got != w.n_lt && lane == 0)
+                        set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
                 }
-                ob = cb;
-                n_lt = m;
-                n_median++;
-                for (uint32_t p = s + lane; p < s + n; p += 32) {
-                    const uint32_t r = S.idx[ob][p];
-                    const float4 lo = S.rlo[r], hi = S.rhi[r];
-                    const float c[3] = {center_of(lo.x, hi.x), center_of(lo.y, hi.y), center_of(lo.z, hi.z)};
-                    grow_keys12(ck, p < s + m, c);
-                    bad |= !box_contains2(win.lt, win.gt, p < s + m, c[0], c[1], c[2]);
-                }
-            }
-            if (__any_sync(kFull, bad) && lane == 0) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
-            warp_reduce_keys12(ck);
-            warp_store_node(O, t.nbase + nd.slot, nd.b, base + s - t.tbase, n, nd.pair, lane);
-            any_split = true;
-            hmax = max(hmax, depth);
-            const uint32_t n_gt = n - n_lt;
-#pragma unroll  // constant c: the child's box and keys stay in registers
-            for (int c = 0; c < 2; ++c) {
-                const uint32_t len = c == 0 ? n_gt : n_lt;
-                const uint32_t cs = c == 0 ? s + n_lt : s;
-                const uint32_t slot = c == 0 ? nd.pair : nd.pair + 1u;
-                const uint32_t pair = c == 0 ? nd.pair + 2u : nd.pair + 2u * n_gt;
-                const uint32_t cdepth = depth + 1u;
-                const float* cbx = c == 0 ? win.gt : win.lt;
-                const uint32_t* cck = c == 0 ? ck + 6 : ck;
-                const bool cleaf =
-                    len <= 1u || cdepth == P.max_depth || (len <= P.max_leaf && len < 2u * P.min_leaf);
-                if (cleaf) {
-                    medium_leaf(S, ob, base, cs, len, slot, cdepth, cbx, t.nbase, t.tbase, P, O, lane);
-                } else if (len > kSmallMax) {
-                    uint32_t li2 = 0;
-                    if (lane == 0) li2 = atomicAdd(&S.list_n[cur ^ 1u], 1u);
-                    li2 = __shfl_sync(kFull, li2, 0);
-                    if (lane == 0) {
-                        MNode& q = S.list[cur ^ 1u][li2];
-                        for (int i = 0; i < 6; ++i) {
-                            q.b[i] = cbx[i];
-                            q.cb[i] = funkey(cck[i]);
-                        }
-                        q.s = cs;
-                        q.n = len;
-                        q.slot = slot;
-                        q.pair = pair;
-                        S.list_x[cur ^ 1u][li2].depth = cdepth;
-                        S.list_x[cur ^ 1u][li2].ib = ob;
+                bad = __any_sync(kFull, side.nan);
+                if (kind != 1u) {
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) {
+                        ck[q] = q < 3 ? warp_min(side.lt[q]) : warp_max(side.lt[q]);
+                        ck[6 + q] = q < 3 ? warp_min(side.gt[q]) : warp_max(side.gt[q]);
                     }
-                } else {
-                    if constexpr (kQueue) {
-                        // the persistent build: listed, and built from shared memory
-                        // once the CTA's own nodes are done
-                        uint32_t ri = 0;
-                        if (lane == 0) ri = atomicAdd(&S.sref_n, 1u);
-                        ri = __shfl_sync(kFull, ri, 0);
+                    if (G > 1u) {
                         if (lane == 0) {
-                            SmallRef& q = S.sref[ri];
-                            for (int i = 0; i < 6; ++i) q.b[i] = cbx[i];
-                            q.slot = slot;
-                            q.pair = pair;
-                            q.depth = cdepth;
-                            q.cs = static_cast<uint16_t>(cs);
-                            q.len = static_cast<uint8_t>(len);
-                            q.ob = static_cast<uint8_t>(ob);
+#pragma unroll
+                            for (int q = 0; q < 12; ++q) {
+                                if (q % 6 < 3)
+                                    atomicMin(&D.keys[q], fkey(ck[q]));
+                                else
+                                    atomicMax(&D.keys[q], fkey(ck[q]));
+                            }
+                            if (bad) D.bad = 1u;
                         }
-                        continue;
-                    }
-                    // subtree of <= 32 objects: write its records back to this task's
-                    // range of the record buffer and queue it for small_kernel
-                    if (lane < len) {
-                        const uint32_t r = S.idx[ob][cs + lane];
-                        Rec rr;
-                        rr.lo = S.rlo[r];
-                        rr.hi = S.rhi[r];
-                        src[cs + lane] = rr;
-                    }
-                    uint32_t si = 0;
-                    if (lane == 0) si = atomicAdd(&O.ctr->n_small, 1u);
-                    si = __shfl_sync(kFull, si, 0);
-                    if (si >= cap_small) {
-                        if (lane == 0) set_error(O.ctr, MGBVH_ERR_CAPACITY, kSiteCapacity);
-                    } else if (lane == 0) {
-                        Task st;
-                        for (int a = 0; a < 3; ++a) {
-                            st.lo[a] = cbx[a];
-                            st.hi[a] = cbx[3 + a];
-                        }
-                        st.start = base + cs;
-                        st.len = len;
-                        st.slot = slot;
-                        st.pair = pair;
-                        st.depth = cdepth;
-                        st.buf = t.buf;
-                        st.tile0 = st.ntiles = 0;
-                        st.nbase = t.nbase;
-                        st.tbase = t.tbase;
-                        small[si] = st;
+                        sync();
+#pragma unroll
+                        for (int q = 0; q < 12; ++q) ck[q] = funkey(D.keys[q]);
+                        bad = D.bad != 0u;
                     }
                 }
             }
+            if (gw) continue;
+            if (kind == 1u)
+                medium_leaf(S, m.ib, base, m.s, m.n, nd.slot, m.depth, nd.b, t.nbase, t.tbase, P, O, lane);
+            else
+                emit(nd, m, w.lt, w.gt, w.n_lt, ck, bad);
         }
         cur ^= 1u;
     }
+    const uint32_t hm = __reduce_max_sync(kFull, hmax);
     if (lane == 0) {
-        if (any_split) atomicMax(&O.ctr->height, hmax);
+        if (hm) atomicMax(&O.ctr->height, hm - 1u);
         if (n_median) atomicAdd(&O.ctr->median_splits, n_median);
     }
     if constexpr (kQueue) {
         // the subtrees of <= 32 objects, one warp each (the loop above ends
         // after a barrier, so the list is complete)
         const uint32_t ns = S.sref_n;
-        for (uint32_t i = warp; i < ns; i += kMediumWarps) {
+        for (uint32_t i = warp; i < ns; i += kW) {
             const SmallRef q = S.sref[i];
             float slo[3] = {0.f, 0.f, 0.f}, shi[3] = {0.f, 0.f, 0.f};
             uint32_t sid = 0;
@@ -2344,47 +2441,35 @@ __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec*
 #ifndef MGBVH_SMALL_TAKE
 #define MGBVH_SMALL_TAKE 1  // 1: small-subtree warps take tasks from a counter (0: grid-stride order)
 #endif
-#ifndef MGBVH_MEDIUM_TAKE
-#define MGBVH_MEDIUM_TAKE 1  // 1: subtree CTAs take tasks from a counter (0: grid-stride order)
-#endif
 
-// The subtree CTA's dynamic shared memory.
-template <bool kLearn, uint32_t kCap>
-constexpr size_t medium_smem_bytes() {
-    return sizeof(MediumSmemT<kCap>);
+// Subtree CTAs per SM that an instance's register budget must allow.
+template <bool kLearn, uint32_t kCap, int kWarps>
+constexpr int medium_ctas() {
+    return kWarps > 4 ? 16 / kWarps : (kLearn ? MGBVH_MEDIUM_LEARN_CTAS : MGBVH_MEDIUM_SMALL_CTAS);
 }
 
-template <bool kLearn, uint32_t kCap>
-__global__ void __launch_bounds__(kMediumThreads, kLearn ? MGBVH_MEDIUM_LEARN_CTAS : MGBVH_MEDIUM_SMALL_CTAS)
-    medium_kernel(const Task* __restrict__ tasks,
-                                                                Rec* rec0, Rec* rec1, Task* small,
-                                                                uint32_t cap_small, Params P, Out O,
-                                                                Learn LN, const uint32_t* range) {
+template <bool kLearn, uint32_t kCap, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, medium_ctas<kLearn, kCap, kWarps>())
+    medium_kernel(const Task* __restrict__ tasks, Rec* rec0, Rec* rec1, Task* small, uint32_t cap_small, Params P,
+                  Out O, Learn LN, const uint32_t* range) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    MediumSmemT<kCap>& S = *reinterpret_cast<MediumSmemT<kCap>*>(smem_raw);
+    MediumSmemT<kCap, kWarps>& S = *reinterpret_cast<MediumSmemT<kCap, kWarps>*>(smem_raw);
     // range (nullable): tasks [range[0], range[1]) instead of all of them
     // (range is ctr->mrange + c for slot chunk c). CTAs take the tasks in
     // turn from a counter (subtree sizes vary, so a fixed assignment leaves
     // a tail): medium_take, or mtake[c] for a chunk.
     const uint32_t t0 = range ? range[0] : 0u;
     const uint32_t n_tasks = range ? range[1] : *reinterpret_cast<volatile uint32_t*>(&O.ctr->n_medium);
-    if (MGBVH_MEDIUM_TAKE) {
-        __shared__ uint32_t s_ti;
-        uint32_t* take = range ? O.ctr->mtake + (range - O.ctr->mrange) : &O.ctr->medium_take;
-        for (;;) {
-            __syncthreads();  // the previous task's readers of s_ti and of S are done
-            if (threadIdx.x == 0) s_ti = t0 + atomicAdd(take, 1u);
-            __syncthreads();
-            const uint32_t ti = s_ti;
-            if (ti >= n_tasks) break;
-            medium_task<kLearn>(S, tasks[ti], rec0, rec1, small, cap_small, P, O, LN);
-        }
-    } else {
-        for (uint32_t ti = t0 + blockIdx.x; ti < n_tasks; ti += gridDim.x) {
-            __syncthreads();
-            medium_task<kLearn>(S, tasks[ti], rec0, rec1, small, cap_small, P, O, LN);
-        }
+    __shared__ uint32_t s_ti;
+    uint32_t* take = range ? O.ctr->mtake + (range - O.ctr->mrange) : &O.ctr->medium_take;
+    for (;;) {
+        __syncthreads();  // the previous task's readers of s_ti and of S are done
+        if (threadIdx.x == 0) s_ti = t0 + atomicAdd(take, 1u);
+        __syncthreads();
+        const uint32_t ti = s_ti;
+        if (ti >= n_tasks) break;
+        medium_task<kLearn>(S, tasks[ti], rec0, rec1, small, cap_small, P, O, LN);
     }
 }
 
@@ -3520,7 +3605,7 @@ void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
 // kernels without a host read in between; the caller checks afterwards that
 // no task was left for a further level (and rebuilds if one was).
 int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, Rec* rec0, Rec* rec1,
-                 bool has_large, uint32_t fixed_levels, uint32_t& launches, uint32_t& levels,
+                 uint32_t n_objects, bool has_large, uint32_t fixed_levels, uint32_t& launches, uint32_t& levels,
                  bool optimistic = false) {
     const cudaStream_t sm = ctx->stream;
     Counters* d_ctr = O.ctr;
@@ -3615,28 +3700,37 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
     if (!fixed_levels) MG_CUDA(cudaEventRecord(ctx->evp[1], sm));
     if (fixed_levels || !ctx->h_ctr->error) {
         // medium subtrees: count read on the device
-        const uint32_t mgrid = std::min<uint32_t>(C.medium, (uint32_t)ctx->sm_count * 4u);
         // subtrees hold at most P.medium_max objects: the smaller-capacity
         // instance leaves room for more CTAs per SM
         // the learned instance only where a subtree node can reach the
         // network's size gate (or samples are collected)
         const bool lrn = (LN.w && LN.min_n <= P.medium_max) || LN.samples,
                    small_cap = P.medium_max <= kMediumSmallCap;
-        const uint32_t mgrid_s =
-            std::min<uint32_t>(C.medium, (uint32_t)ctx->sm_count * (uint32_t)MGBVH_MEDIUM_SMALL_CTAS);
         auto medium = [&](const Task* tasks, const uint32_t* range) {
-            if (lrn && small_cap)
-                launch_k(medium_kernel<true, kMediumSmallCap>, mgrid_s, kMediumThreads, medium_smem_bytes<true, kMediumSmallCap>(), sm,
-                    tasks, rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
+            auto go = [&](auto kernel, size_t smem, int warps, uint32_t per_sm) {
+                launch_k(kernel, std::min<uint32_t>(C.medium, (uint32_t)ctx->sm_count * per_sm), warps * 32, smem, sm, tasks,
+                         rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
+            };
+            // by the objects there are (about 700 per subtree), where each
+            // form is the faster one: subtree phase at 16 / 8 / 4 warps a CTA
+            // 0.059 / 0.074 / 0.121 ms with 65,536 random triangles, 0.090 /
+            // 0.072 / 0.127 with 150,000, 0.166 / 0.106 / 0.129 with 300,000,
+            // 0.296 / 0.182 / 0.166 with 600,000
+            const uint32_t per_sm = n_objects / (range ? kStreamChunks : 1u) / (uint32_t)ctx->sm_count;
+            if (per_sm <= 700u && !lrn)
+                go(medium_kernel<false, kMediumMax, kWidestWarps>, sizeof(MediumSmemT<kMediumMax, kWidestWarps>), kWidestWarps, 1u);
+            else if (per_sm <= 3000u && !lrn)
+                go(medium_kernel<false, kMediumMax, kWideWarps>, sizeof(MediumSmemT<kMediumMax, kWideWarps>), kWideWarps, 2u);
+            else if (per_sm <= 3000u)
+                go(medium_kernel<true, kMediumMax, kWideWarps>, sizeof(MediumSmemT<kMediumMax, kWideWarps>), kWideWarps, 2u);
+            else if (lrn && small_cap)
+                go(medium_kernel<true, kMediumSmallCap, kMediumWarps>, sizeof(MediumSmemT<kMediumSmallCap, kMediumWarps>), kMediumWarps, 5u);
             else if (lrn)
-                launch_k(medium_kernel<true, kMediumMax>, mgrid, kMediumThreads, medium_smem_bytes<true, kMediumMax>(), sm,
-                    tasks, rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
+                go(medium_kernel<true, kMediumMax, kMediumWarps>, sizeof(MediumSmemT<kMediumMax, kMediumWarps>), kMediumWarps, 4u);
             else if (small_cap)
-                launch_k(medium_kernel<false, kMediumSmallCap>, mgrid_s, kMediumThreads, medium_smem_bytes<false, kMediumSmallCap>(), sm,
-                    tasks, rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
+                go(medium_kernel<false, kMediumSmallCap, kMediumWarps>, sizeof(MediumSmemT<kMediumSmallCap, kMediumWarps>), kMediumWarps, 5u);
             else
-                launch_k(medium_kernel<false, kMediumMax>, mgrid, kMediumThreads, medium_smem_bytes<false, kMediumMax>(), sm,
-                    tasks, rec0, rec1, P_<Task>(ctx->small), C.small, P, O, LN, range);
+                go(medium_kernel<false, kMediumMax, kMediumWarps>, sizeof(MediumSmemT<kMediumMax, kMediumWarps>), kMediumWarps, 4u);
         };
         // small subtrees: count read on the device; grid sized for full occupancy
         auto small = ctx->small_warps == 16u ? (subtree_general(P) ? small_kernel<true, 2> : small_kernel<false, 2>)
@@ -3790,7 +3884,7 @@ int run_medians(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, Re
         MG_CUDA(cudaStreamSynchronize(sm));
         if (ctx->h_ctr->error) break;
         uint32_t levels = 0;
-        if ((rc = run_pipeline(ctx, C, P, O, rec0, rec1, ctx->h_ctr->lvl[0][0] > 0, 0, launches, levels)) !=
+        if ((rc = run_pipeline(ctx, C, P, O, rec0, rec1, n_objects, ctx->h_ctr->lvl[0][0] > 0, 0, launches, levels)) !=
             MGBVH_OK)
             return rc;
         MG_CUDA(cudaMemcpyAsync(ctx->h_ctr, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, sm));
@@ -3900,7 +3994,7 @@ int run_build(mgbvh_ctx* ctx, const Input& in, const mgbvh_settings* st, mgbvh_n
     (void)ntiles0;
 
     const bool optimistic = cls == 3 && ctx->levels_hint > 0;
-    if ((rc = run_pipeline(ctx, C, P, O, rec0, rec1, cls == 3, 0, launches, levels, optimistic)) != MGBVH_OK)
+    if ((rc = run_pipeline(ctx, C, P, O, rec0, rec1, n, cls == 3, 0, launches, levels, optimistic)) != MGBVH_OK)
         return rc;
     MG_CUDA(cudaEventRecord(ctx->ev1, sm));
     MG_CUDA(cudaMemcpyAsync(ctx->h_ctr, d_ctr, sizeof(Counters), cudaMemcpyDeviceToHost, sm));
@@ -4217,7 +4311,7 @@ int enqueue_batch(mgbvh_ctx* ctx, const BatchPlan& B, const Caps& C, const mgbvh
         MG_CUDA(cudaGetLastError());
         if (!fixed_levels) MG_CUDA(cudaEventRecord(ctx->evp[0], sm));
         launches = 3;
-        int rc = run_pipeline(ctx, C, P, O, rec0, rec1, B.n_large > 0, fixed_levels, launches, levels);
+        int rc = run_pipeline(ctx, C, P, O, rec0, rec1, n, B.n_large > 0, fixed_levels, launches, levels);
         if (rc != MGBVH_OK) return rc;
     }
     if (!fixed_levels) MG_CUDA(cudaEventRecord(ctx->ev1, sm));
@@ -4640,6 +4734,20 @@ int check_indexed_args(mgbvh_ctx* ctx, const float* v, uint32_t stride, const ui
     return MGBVH_OK;
 }
 
+// The subtree CTA instances' shared-memory limits on the current device.
+template <bool kLearn, uint32_t kCap, int kWarps>
+bool medium_smem_limit() {
+    return cudaFuncSetAttribute(medium_kernel<kLearn, kCap, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(MediumSmemT<kCap, kWarps>)) == cudaSuccess;
+}
+bool medium_smem_limits() {
+    return medium_smem_limit<false, kMediumMax, kMediumWarps>() && medium_smem_limit<true, kMediumMax, kMediumWarps>() &&
+           medium_smem_limit<false, kMediumSmallCap, kMediumWarps>() &&
+           medium_smem_limit<true, kMediumSmallCap, kMediumWarps>() &&
+           medium_smem_limit<false, kMediumMax, kWideWarps>() && medium_smem_limit<true, kMediumMax, kWideWarps>() &&
+           medium_smem_limit<false, kMediumMax, kWidestWarps>();
+}
+
 }  // namespace
 
 extern "C" {
@@ -4676,16 +4784,7 @@ int mgbvh_create(int device, mgbvh_ctx** out_ctx) {
         cudaEventCreate(&ctx->evp[2]) != cudaSuccess ||
         cudaMallocHost(&ctx->h_ctr, sizeof(Counters)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_init, sizeof(Counters)) != cudaSuccess ||
-        cudaFuncSetAttribute(medium_kernel<false, kMediumMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)medium_smem_bytes<false, kMediumMax>()) != cudaSuccess ||
-        cudaFuncSetAttribute(medium_kernel<true, kMediumMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)medium_smem_bytes<true, kMediumMax>()) != cudaSuccess ||
-        cudaFuncSetAttribute(medium_kernel<false, kMediumSmallCap>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)medium_smem_bytes<false, kMediumSmallCap>()) != cudaSuccess ||
-        cudaFuncSetAttribute(medium_kernel<true, kMediumSmallCap>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)medium_smem_bytes<true, kMediumSmallCap>()) != cudaSuccess) {
+        !medium_smem_limits()) {
         mgbvh_destroy(ctx);
         return MGBVH_ERR_CUDA;
     }
@@ -5041,9 +5140,7 @@ int mgbvh_build_aabbs_noalloc(const float* d_aabbs, uint32_t count, const mgbvh_
     void* addr = nullptr;
     int sms = 0;
     if (cudaGetSymbolAddress(&addr, g_noalloc_scratch) != cudaSuccess || !addr) return MGBVH_ERR_CUDA;
-    if (cudaFuncSetAttribute(medium_kernel<false, kMediumMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)medium_smem_bytes<false, kMediumMax>()) != cudaSuccess)
-        return MGBVH_ERR_CUDA;
+    if (!medium_smem_limit<false, kMediumMax, kWidestWarps>()) return MGBVH_ERR_CUDA;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
         return MGBVH_ERR_CUDA;
     NoAllocScratch* S = reinterpret_cast<NoAllocScratch*>(addr);
@@ -5076,7 +5173,8 @@ int mgbvh_build_aabbs_noalloc(const float* d_aabbs, uint32_t count, const mgbvh_
                                                       nullptr, nullptr, S->medium, S->small, O, 0u,
                                                       st->max_depth);
     if (cls == 2)
-        medium_kernel<false, kMediumMax><<<1, kMediumThreads, medium_smem_bytes<false, kMediumMax>(), sm>>>(
+        medium_kernel<false, kMediumMax, kWidestWarps>
+            <<<1, kWidestWarps * 32, sizeof(MediumSmemT<kMediumMax, kWidestWarps>), sm>>>(
             S->medium, S->rec, S->rec, S->small, kNoAllocMax / 2 + 8, P, O, Learn{nullptr, 0, nullptr, 0, nullptr},
             nullptr);
     if (cls != 0) {

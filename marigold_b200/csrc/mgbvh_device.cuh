@@ -183,6 +183,18 @@ __device__ __forceinline__ uint64_t cand_key(float cost, uint32_t axis, uint32_t
     return (static_cast<uint64_t>(fkey(cost)) << 32) | (axis << 8) | idx;
 }
 
+// Minimum and maximum over the warp (one instruction on sm_100a).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Warp-wide minimum of 64-bit keys via two 32-bit reductions.
 __device__ __forceinline__ uint64_t warp_min_key(uint64_t k) {
     const uint32_t hi = static_cast<uint32_t>(k >> 32), lo = static_cast<uint32_t>(k);
@@ -310,6 +322,193 @@ __device__ __forceinline__ void shfl_cand(Cand& c, uint32_t src) {
         c.lt[i] = __shfl_sync(kFull, c.lt[i], src);
         c.gt[i] = __shfl_sync(kFull, c.gt[i], src);
     }
+}
+
+// Bin index of a centroid on one axis of a node, as bin_of gives it. Instead of
+// the divide, the centroid is scaled by bins / ext; the exact form runs only
+// where the scaled value lies within 2^-14 of an integer (the two differ by
+// less than 2^-16: a few roundings of a value below 32), or on axes whose
+// extent or position is extreme.
+struct BinMap {
+    float cmin, ext, cmin2, scale, top;
+    uint32_t bins;
+    bool fast, ok;  // ok: the axis has an extent (bvh/src/lib.rs:339)
+
+    __device__ __forceinline__ BinMap() {}
+    __device__ __forceinline__ BinMap(float cmn, float cmx, uint32_t n_bins) {
+        cmin = cmn;
+        ext = __fsub_rn(cmx, cmn);
+        bins = n_bins;
+        ok = !(ext == 0.0f);
+        fast = ext >= 7.888609052210118e-31f && ext <= 1.2676506002282294e30f && fabsf(cmn) <= 8.507059173023462e37f;
+        cmin2 = __fadd_rn(cmn, cmn);
+        const float b = __uint2float_rn(n_bins);
+        scale = __fdividef(__fmul_rn(b, 0.5f), ext);
+        top = __fsub_rn(b, 0.6f);
+    }
+    __device__ __forceinline__ uint32_t operator()(float lo, float hi) const {
+        // t = scaled value - 0.5 rounds to the integer below the scaled value;
+        // both ends of the range are clamped to a value inside their bin
+        float t = __fmaf_rn(__fsub_rn(__fadd_rn(lo, hi), cmin2), scale, -0.5f);
+        t = fminf(fmaxf(t, -0.4f), top);
+        const float u = __fadd_rn(t, 12582912.0f);  // 1.5 * 2^23: the integer in the low bits
+        const float off = __fsub_rn(t, __fsub_rn(u, 12582912.0f));
+        uint32_t b = __float_as_uint(u) & 31u;
+        if (!fast || fabsf(off) > 0.49993896484375f) b = bin_of(center_of(lo, hi), cmin, ext, bins);
+        return b;
+    }
+};
+
+// Box coordinates as keys for which a larger key is the union: zero is below
+// every key, so cleared bins are empty. Lower bounds: ~fkey; both are two
+// operations each way.
+__device__ __forceinline__ uint32_t key_lo(float f) {
+    const int u = __float_as_int(f);
+    return static_cast<uint32_t>(u ^ (~(u >> 31) & 0x7FFFFFFF));
+}
+__device__ __forceinline__ uint32_t key_hi(float f) {
+    const int u = __float_as_int(f);
+    return static_cast<uint32_t>(u) ^ (static_cast<uint32_t>(u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float unkey_lo(uint32_t k) {
+    const int u = static_cast<int>(k);
+    return __int_as_float(u ^ (~(u >> 31) & 0x7FFFFFFF));
+}
+__device__ __forceinline__ float unkey_hi(uint32_t k) {
+    const int u = static_cast<int>(k);
+    return __uint_as_float(k ^ (static_cast<uint32_t>(~(u >> 31)) | 0x80000000u));
+}
+
+// A node's bins in shared memory: [axis][bin]{count, key_lo xyz, key_hi xyz},
+// cleared to zero; 7 more words after each axis put the 18 sequences of one
+// bin in different banks.
+constexpr uint32_t kSweepAxis = 32u * 7u + 7u;
+constexpr uint32_t kSweepWords = 3u * kSweepAxis;
+
+__device__ __forceinline__ void clear_bins(uint32_t* wb, uint32_t tid, uint32_t nthreads) {
+    for (uint32_t w = tid; w < kSweepWords; w += nthreads) wb[w] = 0u;
+}
+
+// Adds an object to its bins; returns the bins (5 bits per axis).
+__device__ __forceinline__ uint32_t add_to_bins(uint32_t* wb, const BinMap* map, const float4& lo, const float4& hi) {
+    const uint32_t k[6] = {key_lo(lo.x), key_lo(lo.y), key_lo(lo.z), key_hi(hi.x), key_hi(hi.y), key_hi(hi.z)};
+    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    uint32_t code = 0;
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        if (!map[a].ok) continue;  // the same for every object of the node
+        const uint32_t b = map[a](l[a], h[a]);
+        code |= b << (5u * a);
+        uint32_t* w = wb + a * kSweepAxis + b * 7u;
+        atomicAdd(w, 1u);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) atomicMax(w + 1 + i, k[i]);
+    }
+    return code;
+}
+
+struct SweepResult {
+    bool found;
+    uint32_t axis, bin, n_lt, cost;  // cost: its bits
+    float lt[6], gt[6];
+    uint32_t cnt[3];  // objects of bin `lane` on each axis
+};
+
+// One warp: the best binned split of a node of n objects whose bins are wb
+// (evaluate_binned_split over every split index and axis, bvh/src/lib.rs:
+// 255-290, 331-389; first minimum of cost, axis, index). Destroys the boxes
+// in wb, not the counts.
+//
+// The prefix and suffix unions of the 3 x 6 coordinate sequences run
+// sequentially, one lane per sequence with its 32 bins in registers, and pass
+// through wb to the lanes that hold the candidates (lane = split index): 3 x 32
+// shared-memory accesses and 62 maxima, where shuffle scans of every lane's
+// bins take 5 steps of 2 x 7 shuffles per axis.
+__device__ __forceinline__ SweepResult sweep_bins(uint32_t* wb, const BinMap* map, uint32_t n, const NodeArea& area,
+                                                  const Params& P, uint32_t lane) {
+    SweepResult r;
+    uint32_t* const seq = wb + (lane < 18u ? (lane / 6u) * kSweepAxis + 1u + lane % 6u : 0u);
+    uint32_t v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = seq[7 * j];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) r.cnt[a] = wb[a * kSweepAxis + 7u * lane];
+    __syncwarp();
+    // objects in the bins below the lane's, per axis
+    uint32_t below01 = r.cnt[0] | (r.cnt[1] << 16), below2 = r.cnt[2];
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, below01, d), w = __shfl_up_sync(kFull, below2, d);
+        if (lane >= d) {
+            below01 += u;
+            below2 += w;
+        }
+    }
+    below01 -= r.cnt[0] | (r.cnt[1] << 16);
+    below2 -= r.cnt[2];
+    if (lane < 18u) {
+        uint32_t run = v[0];
+#pragma unroll
+        for (int j = 1; j < 32; ++j) {
+            seq[7 * j] = run;
+            run = max(run, v[j]);
+        }
+    }
+    __syncwarp();
+    float sa_lt[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t* w = wb + a * kSweepAxis + 7u * lane + 1u;
+        sa_lt[a] = surface_area(unkey_lo(w[0]), unkey_lo(w[1]), unkey_lo(w[2]), unkey_hi(w[3]), unkey_hi(w[4]),
+                                unkey_hi(w[5]));
+    }
+    __syncwarp();
+    if (lane < 18u) {
+        uint32_t run = v[31];
+#pragma unroll
+        for (int j = 31; j > 0; --j) {
+            seq[7 * j] = run;
+            run = max(run, v[j - 1]);
+        }
+    }
+    __syncwarp();
+    uint32_t best = kNoKey, axis = 3;
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        const uint32_t nl = a == 0 ? below01 & 0xFFFFu : (a == 1 ? below01 >> 16 : below2), ng = n - nl;
+        const uint32_t* w = wb + a * kSweepAxis + 7u * lane + 1u;
+        const float sa_gt = surface_area(unkey_lo(w[0]), unkey_lo(w[1]), unkey_lo(w[2]), unkey_hi(w[3]),
+                                         unkey_hi(w[4]), unkey_hi(w[5]));
+        if (map[a].ok && lane >= 1u && lane < map[a].bins && nl >= P.min_leaf && ng >= P.min_leaf) {
+            // (positive, infinite or the default NaN: the bits order as total_cmp)
+            const uint32_t ck = __float_as_uint(area.split_cost(sa_lt[a], sa_gt, nl, ng));
+            if (ck < best) {
+                best = ck;
+                axis = a;
+            }
+        }
+    }
+    r.cost = __reduce_min_sync(kFull, best);
+    r.found = r.cost != kNoKey;
+    const uint32_t w0 = __ballot_sync(kFull, best == r.cost && axis == 0u),
+                   w1 = __ballot_sync(kFull, best == r.cost && axis == 1u),
+                   w2 = __ballot_sync(kFull, best == r.cost && axis == 2u);
+    r.axis = w0 ? 0u : (w1 ? 1u : 2u);
+    r.bin = r.found ? __ffs(w0 ? w0 : (w1 ? w1 : w2)) - 1u : 1u;
+    const uint32_t nl = r.axis == 0 ? below01 & 0xFFFFu : (r.axis == 1 ? below01 >> 16 : below2);
+    r.n_lt = __shfl_sync(kFull, nl, r.bin);
+    const uint32_t* w = wb + r.axis * kSweepAxis + 7u * r.bin + 1u;
+    uint32_t run = v[0];
+#pragma unroll
+    for (uint32_t j = 1; j < 32u; ++j) run = j < r.bin ? max(run, v[j]) : run;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const uint32_t l = __shfl_sync(kFull, run, r.axis * 6u + i);
+        r.lt[i] = i < 3 ? unkey_lo(l) : unkey_hi(l);
+        r.gt[i] = i < 3 ? unkey_lo(w[i]) : unkey_hi(w[i]);
+    }
+    __syncwarp();
+    return r;
 }
 
 // Segmented reductions over contiguous lane ranges [s, end): shuffle-down
