@@ -43,11 +43,8 @@
 namespace mgbvh {
 
 constexpr uint32_t kMediumMax = 1024;
-#ifndef MGBVH_TILE
-#define MGBVH_TILE 2048  // objects per level-pass tile (tuning knob; a multiple of 256 * the bin batch)
-#endif
-constexpr uint32_t kTile = MGBVH_TILE;
-constexpr int kTileThreads = 256;
+constexpr int kTileThreads = 256;       // threads of a level-pass CTA
+constexpr uint32_t kTileMax = 2560;    // most objects of a level-pass tile (tile_objects)
 #ifndef MGBVH_MEDIUM_WARPS
 #define MGBVH_MEDIUM_WARPS 4  // warps per subtree CTA (tuning knob)
 #endif
@@ -67,7 +64,6 @@ constexpr uint32_t kBinWords = 3 * 32 * 7;  // [axis][bin]{count, lo key xyz, hi
 // slot (L + 2) % 3, last read by level L - 1, is cleared during level L.
 __host__ __device__ __forceinline__ uint32_t lvl_next(uint32_t lv) { return lv == 2u ? 0u : lv + 1u; }
 __host__ __device__ __forceinline__ uint32_t lvl_free(uint32_t lv) { return lv == 0u ? 2u : lv - 1u; }
-constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 struct Rec {
     float4 lo;  // min xyz, object id (bits)
@@ -99,7 +95,7 @@ struct Task {
     float hi[3];
     uint32_t len;
     uint32_t slot, pair, depth, buf;
-    uint32_t tile0, ntiles;
+    uint32_t tile0, cb;  // level-pass nodes: first tile, place of the centroid bound keys
     uint32_t nbase, tbase;  // node-slot and record offsets of the object's mesh (batched builds)
 };
 
@@ -114,35 +110,41 @@ __device__ __forceinline__ Task ldcg_task(const Task* p) {
     return t;
 }
 
+// A tile of a level pass: objects [begin, begin + cnt) of its node.
+struct alignas(16) TileRef {
+    uint32_t task, begin, cnt, pad;
+};
+
 // Split decision of one large node, read by its partition tiles.
 struct Decision {
     uint32_t kind;  // 0 split, 1 leaf (or a forced median deferred to the median passes)
-    uint32_t axis, split_bin, bins;
-    float cmin, ext;
+    uint32_t axis, split_bin;
     uint32_t n_lt;
-    uint32_t child_task[2];  // [0] gt, [1] lt: next-level large task, or kNone
-    uint32_t child_leaf[2];
     uint32_t use_thr;    // 1: a learned proposal won; the partition is centroid < thr
     float thr;
+    uint32_t row;        // tile histogram row with each tile's lt count (tile_hist2 when use_thr)
     uint32_t plain_key;  // cost key of the binned split
     float ltb[6], gtb[6];
 };
 
-// ---------------------------------------------------------------- helpers
+__host__ __device__ __forceinline__ uint32_t tiles_of(uint32_t len, uint32_t tile) { return (len + tile - 1u) / tile; }
 
-// Grows the lt (k[0..5]: min keys xyz, max keys xyz) or gt (k[6..11])
-// centroid key bounds by centroid c; selects with constant indexes keep k in
-// registers.
-__device__ __forceinline__ void grow_keys12(uint32_t* k, bool lt, const float* c) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const uint32_t f = fkey(c[a]);
-        k[a] = lt ? min(k[a], f) : k[a];
-        k[3 + a] = lt ? max(k[3 + a], f) : k[3 + a];
-        k[6 + a] = lt ? k[6 + a] : min(k[6 + a], f);
-        k[9 + a] = lt ? k[9 + a] : max(k[9 + a], f);
+// The tiles of a node of len objects: nt pieces whose sizes differ by at most
+// one (threads tid, tid + step, ... write them).
+__device__ __forceinline__ void write_tiles(TileRef* tiles, uint32_t nt, uint32_t task, uint32_t len, uint32_t tid,
+                                            uint32_t step) {
+    const uint32_t q = len / nt, r = len % nt;
+    for (uint32_t i = tid; i < nt; i += step) {
+        TileRef t;
+        t.task = task;
+        t.begin = i * q + min(i, r);
+        t.cnt = q + (i < r ? 1u : 0u);
+        t.pad = 0;
+        tiles[i] = t;
     }
 }
+
+// ---------------------------------------------------------------- helpers
 
 __device__ __forceinline__ void block_reduce_keys_to_global(uint32_t* keys /*12*/, uint32_t* smem12,
                                                             uint32_t* global12) {
@@ -286,7 +288,7 @@ __device__ __forceinline__ void init_task_bins(uint32_t* b, uint32_t lane, uint3
 // cls: 0 leaf, 1 small, 2 medium, 3 large.
 __global__ void init_root_kernel(uint32_t n, uint32_t cls, uint32_t has_bounds, float b0, float b1,
                                  float b2, float b3, float b4, float b5, Task* large, uint32_t* bins,
-                                 uint32_t* cbkeys, uint32_t* tile_task, uint32_t* tile_begin,
+                                 uint32_t* cbkeys, TileRef* tiles,
                                  Task* medium, Task* small, Out O, uint32_t ntiles,
                                  uint32_t max_depth) {
     pdl_enter();
@@ -310,7 +312,7 @@ __global__ void init_root_kernel(uint32_t n, uint32_t cls, uint32_t has_bounds, 
     t.depth = 0;
     t.buf = 0;
     t.tile0 = 0;
-    t.ntiles = ntiles;
+    t.cb = 0;
     t.nbase = t.tbase = 0;
     if (cls == 0) {
         if (gtid == 0) {
@@ -353,34 +355,22 @@ __global__ void init_root_kernel(uint32_t n, uint32_t cls, uint32_t has_bounds, 
     }
     if (blockIdx.x == 0) init_task_bins(bins, threadIdx.x, blockDim.x);
     if (gtid < 6) cbkeys[gtid] = O.ctr->root_keys[6 + gtid];
-    for (uint32_t i = gtid; i < ntiles; i += gsz) {
-        tile_task[i] = 0;
-        tile_begin[i] = i * kTile;
-    }
+    write_tiles(tiles, ntiles, 0u, n, gtid, gsz);
 }
 
 // ---------------------------------------------------------------- large level
 
-constexpr uint32_t kRecsPerThread = kTile / kTileThreads;  // 8
-
-
 #ifndef MGBVH_BIN_MIN_BLOCKS
-#define MGBVH_BIN_MIN_BLOCKS 4  // CTAs per SM the register budget must allow (tuning knob; 1 / 3 / 4 with batches of 8 / 4 / 4: 682 / 691 / 692 Mtri/s)
+#define MGBVH_BIN_MIN_BLOCKS 4  // bin-pass CTAs per SM the register budget must allow (tuning knob)
 #endif
-#ifndef MGBVH_PART_CODES
-#define MGBVH_PART_CODES 1  // 1: the bin pass stores each record's bins (16 bits) and the partition reads them
-#endif
-constexpr bool kPartCodes = MGBVH_PART_CODES != 0;
 #ifndef MGBVH_BIN_BATCH
-#define MGBVH_BIN_BATCH 4  // records a thread loads before binning them (tuning knob; divides 8)
+#define MGBVH_BIN_BATCH 4  // records a thread loads before binning them (tuning knob)
 #endif
 constexpr uint32_t kBinBatch = MGBVH_BIN_BATCH;
-static_assert(kRecsPerThread % kBinBatch == 0, "the bin batch divides the records per thread");
 #ifndef MGBVH_PART_UNROLL
-#define MGBVH_PART_UNROLL 1  // records in flight per lane in the scatter pass (tuning knob; 1 / 2 / 4: 681 / 676 / 680 Mtri/s)
+#define MGBVH_PART_UNROLL 1  // records in flight per lane in the scatter pass (tuning knob; 2: no faster)
 #endif
 constexpr int kPartUnroll = MGBVH_PART_UNROLL;
-
 
 struct EvalArgs {
     const Task* tasks;
@@ -388,13 +378,11 @@ struct EvalArgs {
     const uint32_t* bins;
     const uint32_t* cbkeys;
     const uint32_t* tile_hist;  // [axis * 32 + bin][tile]: objects of the tile in the axis's bins below bin
-    uint32_t* tile_lt;
     Decision* dec;
     Task* next_tasks;
     uint32_t* next_bins;
-    uint32_t* next_cbkeys;
-    uint32_t* next_tile_task;
-    uint32_t* next_tile_begin;
+    TileRef* next_tiles;
+    uint32_t tile;  // most objects of a tile
     Task* medium;
     Task* small;
     uint32_t cap_tasks, cap_tiles, cap_medium, cap_small;
@@ -410,36 +398,13 @@ struct EvalArgs {
     Task* med;  // nodes waiting for a forced median (cap_tasks entries; count in ctr->n_med)
 };
 
-// Writes the node and its children of a decided split: the per-tile lt
-// counts (exclusive scan across the node's tiles of histogram row `row`:
-// each tile's objects left of the split), the node record, and each child as
-// a leaf, a next-level task, a medium or a small subtree. Each lane scans a
-// contiguous run of the node's tiles (independent loads), runs joined by a
-// warp scan.
+// Writes the node and its children of a decided split, one warp: the node
+// record, and each child as a leaf, a next-level task, a medium or a small
+// subtree. A next-level child's centroid bound keys are those that the
+// partition reduces at its parent's place: 2w for lt, 2w + 1 for gt.
 __device__ void emit_split(const EvalArgs& A, const Params& P, const Out& O, uint32_t w, uint32_t lane,
-                           const Task& t, Decision& d, const uint32_t* hist, uint32_t row) {
+                           const Task& t, const Decision& d) {
     const float nb[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
-    const uint32_t* h = hist + (size_t)row * A.cap_tiles + t.tile0;
-    uint32_t* lt = A.tile_lt + t.tile0;
-    const uint32_t per = (t.ntiles + 31u) >> 5;
-    const uint32_t i0 = min(lane * per, t.ntiles), i1 = min(i0 + per, t.ntiles);
-    uint32_t sum = 0;
-#pragma unroll 8
-    for (uint32_t i = i0; i < i1; ++i) sum += h[i];
-    uint32_t inc = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t u = __shfl_up_sync(kFull, inc, off);
-        if (lane >= static_cast<uint32_t>(off)) inc += u;
-    }
-    const uint32_t total = __shfl_sync(kFull, inc, 31);
-    uint32_t run = inc - sum;
-    for (uint32_t i = i0; i < i1; ++i) {
-        const uint32_t v = h[i];
-        lt[i] = run;
-        run += v;
-    }
-    if (total != d.n_lt && lane == 0) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteCount);
     warp_store_node(O, t.nbase + t.slot, nb, t.start - t.tbase, t.len, t.pair, lane);
     if (lane == 0) atomicMax(&O.ctr->height, t.depth);
     const uint32_t n_gt = t.len - d.n_lt;
@@ -450,9 +415,8 @@ __device__ void emit_split(const EvalArgs& A, const Params& P, const Out& O, uin
     for (int c = 0; c < 2; ++c) {
         const uint32_t len = c == 0 ? n_gt : d.n_lt;
         const uint32_t depth = t.depth + 1u;
-        const bool cleaf = len <= 1u || depth == P.max_depth || (len <= P.max_leaf && len < 2u * P.min_leaf);
-        cls[c] = cleaf ? 0u : (len > P.medium_max ? 1u : (len > kSmallMax ? 2u : 3u));
-        ntl[c] = cls[c] == 1u ? (len + kTile - 1) / kTile : 0u;
+        cls[c] = leaf_rule(len, depth, P) ? 0u : (len > P.medium_max ? 1u : (len > kSmallMax ? 2u : 3u));
+        ntl[c] = cls[c] == 1u ? tiles_of(len, A.tile) : 0u;
     }
     uint32_t slot_task = 0, slot_tile = 0, slot_med = 0, slot_small = 0;
     if (lane == 0) {
@@ -488,14 +452,13 @@ __device__ void emit_split(const EvalArgs& A, const Params& P, const Out& O, uin
         ct.pair = pair;
         ct.depth = depth;
         ct.buf = t.buf ^ 1u;
-        ct.tile0 = ct.ntiles = 0;
+        ct.tile0 = ct.cb = 0;
         ct.nbase = t.nbase;
         ct.tbase = t.tbase;
         // this child's place in its list: after the gt child when both share it
         const uint32_t before = (c == 1 && cls[0] == cls[1]) ? 1u : 0u;
         if (cls[c] == 0u) {
             warp_store_node(O, t.nbase + slot, cb, start - t.tbase, len, 0u, lane);
-            d.child_leaf[c] = 1;
             if (lane == 0 && len > 1) {
                 atomicAdd(&O.ctr->holes, 1u);
                 if (depth == P.max_depth) atomicAdd(&O.ctr->depth_capped, 1u);
@@ -509,15 +472,10 @@ __device__ void emit_split(const EvalArgs& A, const Params& P, const Out& O, uin
                 continue;
             }
             ct.tile0 = t0;
-            ct.ntiles = nt;
+            ct.cb = 2u * w + (c == 0 ? 1u : 0u);
             if (lane == 0) A.next_tasks[ti] = ct;
             init_task_bins(A.next_bins + (size_t)ti * kBinWords, lane, 32);
-            if (lane < 6) A.next_cbkeys[6 * ti + lane] = lane < 3 ? kKeyPosInf : kKeyNegInf;
-            for (uint32_t i = lane; i < nt; i += 32) {
-                A.next_tile_task[t0 + i] = ti;
-                A.next_tile_begin[t0 + i] = i * kTile;
-            }
-            d.child_task[c] = ti;
+            write_tiles(A.next_tiles + t0, nt, ti, len, lane, 32);
         } else if (cls[c] == 2u) {
             const uint32_t mi = slot_med + before;
             if (mi >= A.cap_medium) {
@@ -534,7 +492,29 @@ __device__ void emit_split(const EvalArgs& A, const Params& P, const Out& O, uin
             if (lane == 0) A.small[si] = ct;
         }
     }
-    if (lane == 0) A.dec[w] = d;
+}
+
+// A large node that stays a leaf, one warp (the partition places its objects).
+__device__ __forceinline__ void emit_leaf(const Params& P, const Out& O, uint32_t lane, const Task& t) {
+    const float nb[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
+    warp_store_node(O, t.nbase + t.slot, nb, t.start - t.tbase, t.len, 0u, lane);
+    if (lane == 0 && t.len > 1) {
+        atomicAdd(&O.ctr->holes, 1u);
+        if (t.depth == P.max_depth) atomicAdd(&O.ctr->depth_capped, 1u);
+    }
+}
+
+// A large node without a binned split and with too many objects for a leaf:
+// the forced median (bvh/src/lib.rs:527-531) runs in the median passes after
+// this build's pipeline. The partition treats the node as a leaf: it only
+// copies the ids into the permutation, which the leaves of the node's subtree
+// overwrite later. One lane.
+__device__ __forceinline__ void queue_median(const EvalArgs& A, const Out& O, const Task& t) {
+    const uint32_t mi = atomicAdd(&O.ctr->n_med, 1u);
+    if (mi < A.cap_tasks)
+        A.med[mi] = t;
+    else
+        set_error(O.ctr, MGBVH_ERR_CAPACITY, kSiteCapacity);
 }
 
 // transposed network parameters as 16-byte vectors (the learned evaluation
@@ -543,9 +523,8 @@ constexpr uint32_t kEvalWeightVec = mgbvh_mlp::kTParams * 2u / 16u;
 static_assert(mgbvh_mlp::kTParams * 2u % 16u == 0u, "the transposed parameters are whole 16-byte vectors");
 constexpr size_t kEvalWeightBytes = mgbvh_mlp::kTParams * 2u;
 
-// kLearn: with the learned form's network (a separate instantiation keeps
-// the plain evaluation's code small: a cold kernel fetches every instruction).
-template <bool kLearn>
+// The evaluation of one node by one warp as a pass of its own: the learned form
+// and sample output (plain builds evaluate in the partition's CTAs).
 __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint32_t w, uint32_t lane) {
     const Task t = A.tasks[w];
     const uint32_t* tb = A.bins + (size_t)w * kBinWords;
@@ -553,8 +532,8 @@ __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint
     float cmn[3], ext[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        cmn[a] = funkey(A.cbkeys[6 * w + a]);
-        ext[a] = __fsub_rn(funkey(A.cbkeys[6 * w + 3 + a]), cmn[a]);
+        cmn[a] = funkey(A.cbkeys[6 * t.cb + a]);
+        ext[a] = __fsub_rn(funkey(A.cbkeys[6 * t.cb + 3 + a]), cmn[a]);
     }
     const float nb[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
     const uint32_t B = P.bins ? P.bins : 32u;
@@ -562,11 +541,8 @@ __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint
     Decision d;
     d.kind = 1;
     d.axis = d.split_bin = 0;
-    d.bins = B;
-    d.cmin = d.ext = 0.0f;
     d.n_lt = 0;
-    d.child_task[0] = d.child_task[1] = kNone;
-    d.child_leaf[0] = d.child_leaf[1] = 0;
+    d.row = 0;
     d.use_thr = 0;
     d.thr = 0.0f;
     d.plain_key = kNoKey;
@@ -588,19 +564,9 @@ __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint
         const uint32_t wlo = static_cast<uint32_t>(wk);
         if (wlo == kNoKey) {
             if (t.len > P.max_leaf) {
-                // no binned split and too many objects for a leaf: the forced
-                // median (bvh/src/lib.rs:527-531) runs in the median passes
-                // after this build's pipeline. The partition treats the node
-                // as a leaf: it only copies the ids into the permutation, which
-                // the leaves of the node's subtree overwrite later.
                 if (lane == 0) {
-                    d.kind = 1;
                     A.dec[w] = d;
-                    const uint32_t mi = atomicAdd(&O.ctr->n_med, 1u);
-                    if (mi < A.cap_tasks)
-                        A.med[mi] = t;
-                    else
-                        set_error(O.ctr, MGBVH_ERR_CAPACITY, kSiteCapacity);
+                    queue_median(A, O, t);
                 }
                 return;
             }
@@ -616,29 +582,22 @@ __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint
         }
     }
     if (leaf) {
-        warp_store_node(O, t.nbase + t.slot, nb, t.start - t.tbase, t.len, 0u, lane);
-        if (lane == 0) {
-            A.dec[w] = d;
-            if (t.len > 1) {
-                atomicAdd(&O.ctr->holes, 1u);
-                if (t.depth == P.max_depth) atomicAdd(&O.ctr->depth_capped, 1u);
-            }
-        }
+        emit_leaf(P, O, lane, t);
+        if (lane == 0) A.dec[w] = d;
         return;
     }
     d.kind = 0;
-    d.cmin = sel3(cmn, d.axis);
-    d.ext = sel3(ext, d.axis);
     d.n_lt = win.n_lt;
+    d.row = d.axis * 32u + d.split_bin;
     for (int i = 0; i < 6; ++i) {
         d.ltb[i] = win.lt[i];
         d.gtb[i] = win.gt[i];
     }
-    if (kLearn && A.lw && B == 32u && t.len >= A.lmin_n) {
+    if (A.lw && B == 32u && t.len >= A.lmin_n) {
         // the learned form: run the network; with proposals to score, the
         // decision waits for the refine pass (lvl_eval2_kernel)
-        const float cb[6] = {cmn[0], cmn[1], cmn[2], funkey(A.cbkeys[6 * w + 3]),
-                             funkey(A.cbkeys[6 * w + 4]), funkey(A.cbkeys[6 * w + 5])};
+        const float cb[6] = {cmn[0], cmn[1], cmn[2], funkey(A.cbkeys[6 * t.cb + 3]),
+                             funkey(A.cbkeys[6 * t.cb + 4]), funkey(A.cbkeys[6 * t.cb + 5])};
         float f[24];
         node_features(nb, cb, t.len, t.depth, cnt, f);
         int top0 = 0, top1 = 0;
@@ -663,107 +622,93 @@ __device__ void eval_task(const EvalArgs& A, const Params& P, const Out& O, uint
             return;
         }
     }
-    emit_split(A, P, O, w, lane, t, d, A.tile_hist, d.axis * 32u + d.split_bin);
+    emit_split(A, P, O, w, lane, t, d);
+    if (lane == 0) A.dec[w] = d;
 }
 
-template <bool kLearn>
 __global__ void __launch_bounds__(128) lvl_eval_kernel(EvalArgs A, Params P, Out O) {
     pdl_enter();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n_tasks = O.ctr->lvl[A.lv][0];
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    if constexpr (kLearn) {
-        // the network's parameters staged in shared memory by the whole CTA
-        // (19.8 KB, coalesced), so each forward pass reads them at shared-memory
-        // latency instead of one dependent L2 round trip per group of inputs
-        extern __shared__ __align__(16) unsigned char eval_dsm[];
-        if (blockIdx.x * (blockDim.x >> 5) >= n_tasks) return;  // block-uniform: no node here
-        if (A.lw) {
-            const uint4* gw = reinterpret_cast<const uint4*>(A.lw);
-            uint4* sw = reinterpret_cast<uint4*>(eval_dsm);
-            for (uint32_t i = threadIdx.x; i < kEvalWeightVec; i += blockDim.x) sw[i] = gw[i];
-            __syncthreads();
-            A.lw = reinterpret_cast<const __nv_bfloat16*>(eval_dsm);
-        }
+    // the network's parameters staged in shared memory by the whole CTA
+    // (19.8 KB, coalesced), so each forward pass reads them at shared-memory
+    // latency instead of one dependent L2 round trip per group of inputs
+    extern __shared__ __align__(16) unsigned char eval_dsm[];
+    if (blockIdx.x * (blockDim.x >> 5) >= n_tasks) return;  // block-uniform: no node here
+    if (A.lw) {
+        const uint4* gw = reinterpret_cast<const uint4*>(A.lw);
+        uint4* sw = reinterpret_cast<uint4*>(eval_dsm);
+        for (uint32_t i = threadIdx.x; i < kEvalWeightVec; i += blockDim.x) sw[i] = gw[i];
+        __syncthreads();
+        A.lw = reinterpret_cast<const __nv_bfloat16*>(eval_dsm);
     }
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n_tasks; w += nwarps)
-        eval_task<kLearn>(A, P, O, w, lane);
+        eval_task(A, P, O, w, lane);
 }
 
 // Per-tile bin histograms (count + AABB per axis and bin) of the large nodes
 // with shared-memory atomics, merged into the node's global bins. Grid-stride over
 // the level's tiles; the tile count is read on the device. Each thread loads
-// its records of the tile first (kTile / kTileThreads of them), then bins
-// them. Also clears the level counter slot two levels ahead (the previous
-// level's kernels, which read it, have finished; the next writer is the
-// next level's evaluation). Each record's bin on every axis (5 bits each)
-// goes to `codes` at its position, for the partition pass.
+// kBinBatch of its records at a time, then bins them. Also clears the level
+// counter slot two levels ahead (the previous level's kernels, which read it,
+// have finished; the next writer is this level's partition) and the node's
+// place for its children's centroid bounds. Each record's bin on every axis (5
+// bits each) goes to `codes` at its position, for the partition pass.
+// What bounds it: the shared-memory atomics (21 per record), whose lanes take
+// turns where they share a bin. So the axes on which a warp's first records do
+// (meshes with runs of neighbours in order) read the bin first (add_to_bins):
+// 131 -> 75 us for 4.2M objects of the mixed scene, half of it in such runs
+// (8.6 turns per atomic before); in meshes without them the look at the first
+// records costs 1%, while reading first always would cost 6%.
 __global__ void __launch_bounds__(kTileThreads, MGBVH_BIN_MIN_BLOCKS) lvl_bin_kernel(
-    const Task* __restrict__ tasks, const uint32_t* __restrict__ cbkeys, uint32_t* __restrict__ bins,
-    const uint32_t* __restrict__ tile_task, const uint32_t* __restrict__ tile_begin,
-    uint32_t* __restrict__ tile_hist, uint32_t cap_tiles, const Rec* __restrict__ rec0,
-    const Rec* __restrict__ rec1, uint16_t* __restrict__ codes, Counters* __restrict__ ctr, uint32_t lv,
-    Params P) {
+    const Task* __restrict__ tasks, const uint32_t* __restrict__ cbkeys, uint32_t* __restrict__ next_cbkeys,
+    uint32_t* __restrict__ bins, const TileRef* __restrict__ tiles, uint32_t* __restrict__ tile_hist,
+    uint32_t cap_tiles, const Rec* __restrict__ rec0, const Rec* __restrict__ rec1, uint16_t* __restrict__ codes,
+    Counters* __restrict__ ctr, uint32_t lv, Params P) {
     pdl_enter();
-    __shared__ uint32_t sb[kBinWords];
+    __shared__ uint32_t sb[kSweepWords];
     if (blockIdx.x == 0 && threadIdx.x < 2) ctr->lvl[lvl_free(lv)][threadIdx.x] = 0;
     const uint32_t ntiles = ctr->lvl[lv][1];
     const uint32_t B = P.bins ? P.bins : 32u;
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         __syncthreads();
-        init_task_bins(sb, threadIdx.x, blockDim.x);
-        const uint32_t ti = tile_task[tile];
-        const Task& t = tasks[ti];
-        const uint32_t begin = tile_begin[tile];
-        const uint32_t cnt = min(kTile, t.len - begin);
-        const Rec* src = (t.buf ? rec1 : rec0) + t.start + begin;
-        float cmn[3], ext[3];
+        clear_bins(sb, threadIdx.x, kTileThreads);
+        const TileRef tr = tiles[tile];
+        const Task& t = tasks[tr.task];
+        const uint32_t cnt = tr.cnt, first = t.start + tr.begin;
+        const Rec* src = (t.buf ? rec1 : rec0) + first;
+        const uint32_t* ck = cbkeys + 6 * t.cb;
+        BinMap map[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            cmn[a] = funkey(cbkeys[6 * ti + a]);
-            ext[a] = __fsub_rn(funkey(cbkeys[6 * ti + 3 + a]), cmn[a]);
-        }
-        // records loaded kBinBatch at a time, then binned
-#pragma unroll
-        for (uint32_t k0 = 0; k0 < kRecsPerThread; k0 += kBinBatch) {
+        for (int a = 0; a < 3; ++a) map[a] = BinMap(funkey(ck[a]), funkey(ck[3 + a]), B);
+        if (tr.begin == 0u && threadIdx.x < 12)
+            next_cbkeys[12 * tr.task + threadIdx.x] = (threadIdx.x % 6) < 3 ? kKeyPosInf : kKeyNegInf;
+        __syncthreads();  // the tile's bins are cleared
+        uint32_t dense = 8u;  // axes on which the warp's lanes share bins (8: not looked at yet)
+        for (uint32_t k0 = threadIdx.x - lane; k0 < cnt; k0 += kBinBatch * kTileThreads) {
             float4 rl[kBinBatch], rh[kBinBatch];
 #pragma unroll
             for (uint32_t k = 0; k < kBinBatch; ++k) {
-                const uint32_t i = threadIdx.x + (k0 + k) * kTileThreads;
+                const uint32_t i = k0 + k * kTileThreads + lane;
                 if (i < cnt) {
                     rl[k] = src[i].lo;
                     rh[k] = src[i].hi;
                 }
             }
-            if (k0 == 0) __syncthreads();  // the tile's bins are initialized
+            if (dense == 8u) dense = shared_bins(map, rl[0], rh[0], k0 + lane < cnt);
 #pragma unroll
             for (uint32_t k = 0; k < kBinBatch; ++k) {
-                const uint32_t i = threadIdx.x + (k0 + k) * kTileThreads;
-                if (i >= cnt) break;
-                const float l[3] = {rl[k].x, rl[k].y, rl[k].z}, h[3] = {rh[k].x, rh[k].y, rh[k].z};
-                uint32_t code = 0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (ext[a] == 0.0f) continue;  // block-uniform
-                    const uint32_t b = bin_of(center_of(l[a], h[a]), cmn[a], ext[a], B);
-                    code |= b << (5 * a);
-                    uint32_t* w = sb + (a * 32 + b) * 7;
-                    atomicAdd(w, 1u);
-                    atomicMin(w + 1, fkey(l[0]));
-                    atomicMin(w + 2, fkey(l[1]));
-                    atomicMin(w + 3, fkey(l[2]));
-                    atomicMax(w + 4, fkey(h[0]));
-                    atomicMax(w + 5, fkey(h[1]));
-                    atomicMax(w + 6, fkey(h[2]));
-                }
-                if (kPartCodes) codes[t.start + begin + i] = static_cast<uint16_t>(code);
+                const uint32_t i = k0 + k * kTileThreads + lane;
+                if (i < cnt) codes[first + i] = static_cast<uint16_t>(add_to_bins(sb, map, rl[k], rh[k], dense));
             }
         }
         __syncthreads();
         if (threadIdx.x < 96) {
             // per axis (one warp each): the tile's count of objects in the
             // bins below each bin, an exclusive scan over the 32 bins
-            const uint32_t lane = threadIdx.x & 31u, c = sb[threadIdx.x * 7];
+            const uint32_t c = sb[(threadIdx.x >> 5) * kSweepAxis + lane * 7u];
             uint32_t inc = c;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
@@ -772,17 +717,17 @@ __global__ void __launch_bounds__(kTileThreads, MGBVH_BIN_MIN_BLOCKS) lvl_bin_ke
             }
             tile_hist[(size_t)threadIdx.x * cap_tiles + tile] = inc - c;
         }
-        uint32_t* gb = bins + (size_t)ti * kBinWords;
-        for (uint32_t k = threadIdx.x; k < kBinWords; k += blockDim.x) {
+        uint32_t* gb = bins + (size_t)tr.task * kBinWords;
+        for (uint32_t k = threadIdx.x; k < kBinWords; k += kTileThreads) {
             const uint32_t bin = k / 7u, f = k % 7u;
-            const uint32_t v = sb[k];
-            if (sb[bin * 7] == 0) continue;
+            const uint32_t* w = sb + bin * 7u + (bin >> 5) * 7u;  // (an axis's 32 bins, then 7 spare words)
+            if (w[0] == 0u) continue;
             if (f == 0)
-                atomicAdd(gb + k, v);
+                atomicAdd(gb + k, w[0]);
             else if (f <= 3)
-                atomicMin(gb + k, v);
+                atomicMin(gb + k, ~w[f]);  // key_lo is the complement of the global key
             else
-                atomicMax(gb + k, v);
+                atomicMax(gb + k, w[f]);
         }
     }
 }
@@ -796,8 +741,8 @@ __global__ void __launch_bounds__(kTileThreads, MGBVH_BIN_MIN_BLOCKS) lvl_bin_ke
 // bins outside [2q - 1, 2q + 2] are at least ext / 32 away from them, far
 // more than the rounding of the bin index (a few ulps of ext) and of the
 // thresholds (an ulp of the coordinates), as long as the coordinates are
-// within 2^14 extents of the origin; else (or without bin codes) the window
-// is every bin and every object is compared, as before.
+// within 2^14 extents of the origin; else the window is every bin and every
+// object is compared.
 #ifndef MGBVH_REFINE_WINDOW
 #define MGBVH_REFINE_WINDOW 1  // 0: the refine pass compares every object (no coarse-bin window)
 #endif
@@ -811,7 +756,7 @@ constexpr uint32_t kRefineBatch = MGBVH_REFINE_BATCH;
 
 __device__ __forceinline__ bool refine_window(float cmin, float ext, uint32_t q, uint32_t& lo, uint32_t& hi) {
     const float cmax = __fadd_rn(cmin, ext);
-    const bool ok = MGBVH_REFINE_WINDOW && kPartCodes && ext > 0.0f && ext < 3.0e38f &&
+    const bool ok = MGBVH_REFINE_WINDOW && ext > 0.0f && ext < 3.0e38f &&
                     fabsf(cmin) <= __fmul_rn(ext, 16384.0f) &&
                     fabsf(cmax) <= __fmul_rn(ext, 16384.0f);
     lo = ok && q > 0u ? 2u * q - 1u : 0u;
@@ -830,8 +775,7 @@ __device__ __forceinline__ bool refine_window(float cmin, float ext, uint32_t q,
 __global__ void __launch_bounds__(kTileThreads, MGBVH_REFINE_MIN_BLOCKS) lvl_refine_bin_kernel(
     const Task* __restrict__ tasks, const uint32_t* __restrict__ cbkeys,
     const LvlRefine* __restrict__ refine, uint32_t* __restrict__ rbins,
-    const uint32_t* __restrict__ tile_task, const uint32_t* __restrict__ tile_begin,
-    uint32_t* __restrict__ tile_hist2, const uint32_t* __restrict__ tile_hist, uint32_t cap_tiles,
+    const TileRef* __restrict__ tiles, uint32_t* __restrict__ tile_hist2, const uint32_t* __restrict__ tile_hist, uint32_t cap_tiles,
     const Rec* __restrict__ rec0, const Rec* __restrict__ rec1, const uint16_t* __restrict__ codes,
     const Counters* __restrict__ ctr, uint32_t lv) {
     pdl_enter();
@@ -839,7 +783,8 @@ __global__ void __launch_bounds__(kTileThreads, MGBVH_REFINE_MIN_BLOCKS) lvl_ref
     __shared__ float sthr[32];
     const uint32_t ntiles = ctr->lvl[lv][1];
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t ti = tile_task[tile];
+        const TileRef tr = tiles[tile];
+        const uint32_t ti = tr.task;
         const LvlRefine R = refine[ti];
         if (!R.on) continue;  // block-uniform
         __syncthreads();      // the previous tile's readers of sb are done
@@ -847,29 +792,27 @@ __global__ void __launch_bounds__(kTileThreads, MGBVH_REFINE_MIN_BLOCKS) lvl_ref
             const uint32_t f7 = i % 7u;
             sb[i] = f7 == 0 ? 0u : (f7 <= 3 ? kKeyPosInf : kKeyNegInf);
         }
+        const Task& t = tasks[ti];
         uint32_t ax[2], wlo[2], whi[2];
         bool act[2];
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
             ax[p] = min(R.prop[p] >> 4, 2u);
-            const float cmin = funkey(cbkeys[6 * ti + ax[p]]);
-            const float ext = __fsub_rn(funkey(cbkeys[6 * ti + 3 + ax[p]]), cmin);
+            const float cmin = funkey(cbkeys[6 * t.cb + ax[p]]);
+            const float ext = __fsub_rn(funkey(cbkeys[6 * t.cb + 3 + ax[p]]), cmin);
             act[p] = ext > 0.0f;
             refine_window(cmin, ext, R.prop[p] & 15u, wlo[p], whi[p]);
             if (threadIdx.x >= 16u * p && threadIdx.x < 16u * (p + 1))
                 sthr[threadIdx.x] = proposal_threshold(cmin, ext, R.prop[p] & 15u, threadIdx.x & 15u);
         }
         __syncthreads();
-        const Task& t = tasks[ti];
-        const uint32_t begin = tile_begin[tile];
-        const uint32_t cnt = min(kTile, t.len - begin);
+        const uint32_t begin = tr.begin, cnt = tr.cnt;
         const Rec* src = (t.buf ? rec1 : rec0) + t.start + begin;
         const uint16_t* cs = codes + t.start + begin;
         const bool all0 = wlo[0] == 0u && whi[0] == 31u, all1 = wlo[1] == 0u && whi[1] == 31u;
         // batches of kRefineBatch objects per thread: their codes loaded
         // together, then the records of those inside a window, then compared
-#pragma unroll
-        for (uint32_t j0 = 0; j0 < kRecsPerThread; j0 += kRefineBatch) {
+        for (uint32_t j0 = 0; j0 * kTileThreads < cnt; j0 += kRefineBatch) {
             uint32_t code[kRefineBatch];
 #pragma unroll
             for (uint32_t q = 0; q < kRefineBatch; ++q) {
@@ -963,8 +906,8 @@ __device__ void eval2_task(const EvalArgs& A, const Params& P, const Out& O, uin
     const LvlRefine R = A.refine[w];
     const uint32_t p = lane >> 4, k = lane & 15u;
     const uint32_t a = min(R.prop[p] >> 4, 2u);
-    const float cmin = funkey(A.cbkeys[6 * w + a]);
-    const float ext = __fsub_rn(funkey(A.cbkeys[6 * w + 3 + a]), cmin);
+    const float cmin = funkey(A.cbkeys[6 * t.cb + a]);
+    const float ext = __fsub_rn(funkey(A.cbkeys[6 * t.cb + 3 + a]), cmin);
     const float thr = proposal_threshold(cmin, ext, R.prop[p] & 15u, k);
     const uint32_t* rb = A.rbins + (size_t)w * kRBinWords + p * 17u * 7u;
     float lt[6], gt[6];
@@ -1055,10 +998,10 @@ __device__ void eval2_task(const EvalArgs& A, const Params& P, const Out& O, uin
             d.gtb[i] = __shfl_sync(kFull, gt[i], src);
         }
         if (lane == 0) atomicAdd(&O.ctr->learned, 1u);
-        emit_split(A, P, O, w, lane, t, d, A.tile_hist2, (src >> 4) * 17u + (src & 15u));
-    } else {
-        emit_split(A, P, O, w, lane, t, d, A.tile_hist, d.axis * 32u + d.split_bin);
+        d.row = (src >> 4) * 17u + (src & 15u);
     }
+    emit_split(A, P, O, w, lane, t, d);
+    if (lane == 0) A.dec[w] = d;
 }
 
 __global__ void __launch_bounds__(128) lvl_eval2_kernel(EvalArgs A, Params P, Out O) {
@@ -1186,7 +1129,7 @@ __global__ void __launch_bounds__(256) lvl_sample_kernel(const Task* __restrict_
                 }
             }
             float cb[6];
-            for (int a = 0; a < 6; ++a) cb[a] = funkey(cbkeys[6 * w + a]);
+            for (int a = 0; a < 6; ++a) cb[a] = funkey(cbkeys[6 * t.cb + a]);
             uint32_t cnt[3];
             for (int a = 0; a < 3; ++a)
                 cnt[a] = cb[3 + a] - cb[a] == 0.0f ? 0u : bins[(size_t)w * kBinWords + (a * 32 + lane) * 7];
@@ -1201,156 +1144,310 @@ __global__ void __launch_bounds__(256) lvl_sample_kernel(const Task* __restrict_
     }
 }
 
+// A partition CTA's shared memory.
+struct PartSmem {
+    uint32_t bins[kSweepWords];  // the node's bins; then the unions of the bins from each bin on
+    uint32_t pre[kSweepWords];   // the unions of the bins below each bin
+    uint32_t cost[3], bin[3], n_lt[3];  // each axis's best split
+    Decision d;
+    uint32_t wcnt[kTileThreads / 32];
+    uint32_t lt_off;  // lt objects of the node's earlier tiles
+    uint32_t keys[12];
+    uint32_t bad;
+};
+
+// The CTA of a tile decides its node's split (evaluate_binned_split over every
+// axis and index, bvh/src/lib.rs:255-290, 331-389; first minimum of cost, axis,
+// index): every tile's CTA does so for itself, in about 3 us, where a launch of
+// its own with one warp per node took 10 us a level. 4 threads per coordinate
+// sequence and direction scan its 32 bins (8 each), then one warp per axis
+// prices the candidates, a bin each. Level passes on 65,536 random triangles
+// 0.162 -> 0.112 ms, on 4,096 0.068 -> 0.047 ms.
+__device__ __forceinline__ void part_decide(PartSmem& S, const EvalArgs& A, const Task& t, uint32_t ti,
+                                            const Params& P) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t* gb = A.bins + (size_t)ti * kBinWords;
+    for (uint32_t k = tid; k < kBinWords; k += kTileThreads) {
+        const uint32_t bin = k / 7u, f = k % 7u, v = gb[k];
+        S.bins[k + (bin >> 5) * 7u] = (f >= 1u && f <= 3u) ? ~v : v;  // lower bounds as key_lo
+    }
+    __syncthreads();
+    uint32_t v[8];
+    const uint32_t q = tid >> 2, chunk = tid & 3u, sq = q < 18u ? q : q - 18u;
+    const bool fwd = q < 18u, scan = tid < 144u;
+    const uint32_t at = (sq / 6u) * kSweepAxis + 1u + sq % 6u;
+    if (scan) {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) v[j] = S.bins[at + 7u * (fwd ? 8u * chunk + j : 31u - 8u * chunk - j)];
+    }
+    uint32_t cnt = 0;
+    if (warp < 3u) cnt = S.bins[warp * kSweepAxis + 7u * lane];
+    __syncthreads();
+    if (tid < 160u) {  // whole warps
+        uint32_t run = 0;
+        if (scan) {
+            run = v[0];
+#pragma unroll
+            for (uint32_t j = 1; j < 8; ++j) run = max(run, v[j]);
+        }
+        // union of the chunks before this one
+        uint32_t ex = __shfl_up_sync(kFull, run, 1, 4);
+        if (chunk == 0u) ex = 0u;
+        const uint32_t e2 = __shfl_up_sync(kFull, ex, 1, 4);
+        if (chunk >= 1u) ex = max(ex, e2);
+        const uint32_t e3 = __shfl_up_sync(kFull, ex, 2, 4);
+        if (chunk >= 2u) ex = max(ex, e3);
+        if (scan) {
+            run = ex;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                if (fwd) {
+                    S.pre[at + 7u * (8u * chunk + j)] = run;  // bins below this one
+                    run = max(run, v[j]);
+                } else {
+                    run = max(run, v[j]);
+                    S.bins[at + 7u * (31u - 8u * chunk - j)] = run;  // this bin and those above
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (warp < 3u) {
+        const uint32_t a = warp;
+        uint32_t inc = cnt;
+#pragma unroll
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(kFull, inc, d);
+            if (lane >= d) inc += u;
+        }
+        const uint32_t nl = inc - cnt, ng = t.len - nl;
+        const float nb[6] = {t.lo[0], t.lo[1], t.lo[2], t.hi[0], t.hi[1], t.hi[2]};
+        const NodeArea area(nb);
+        const uint32_t B = P.bins ? P.bins : 32u;
+        const uint32_t* ck = A.cbkeys + 6 * t.cb;
+        const bool ok = !(__fsub_rn(funkey(ck[3 + a]), funkey(ck[a])) == 0.0f);
+        uint32_t best = kNoKey;
+        if (ok && lane >= 1u && lane < B && nl >= P.min_leaf && ng >= P.min_leaf) {
+            const uint32_t *l = S.pre + a * kSweepAxis + 7u * lane + 1u, *g = S.bins + a * kSweepAxis + 7u * lane + 1u;
+            best = __float_as_uint(area.split_cost(
+                surface_area(unkey_lo(l[0]), unkey_lo(l[1]), unkey_lo(l[2]), unkey_hi(l[3]), unkey_hi(l[4]),
+                             unkey_hi(l[5])),
+                surface_area(unkey_lo(g[0]), unkey_lo(g[1]), unkey_lo(g[2]), unkey_hi(g[3]), unkey_hi(g[4]),
+                             unkey_hi(g[5])),
+                nl, ng));
+        }
+        const uint32_t low = __reduce_min_sync(kFull, best);
+        const uint32_t win = __ffs(__ballot_sync(kFull, best == low)) - 1u;
+        if (lane == win) {
+            S.cost[a] = low;
+            S.bin[a] = lane;
+            S.n_lt[a] = nl;
+        }
+    }
+    __syncthreads();
+    if (tid < 6u || tid == 32u) {
+        const uint32_t c0 = S.cost[0], c1 = S.cost[1], c2 = S.cost[2];
+        const uint32_t low = min(c0, min(c1, c2));
+        const uint32_t a = c0 == low ? 0u : (c1 == low ? 1u : 2u), b = S.bin[a];
+        if (tid < 6u) {
+            const uint32_t w = a * kSweepAxis + 7u * b + 1u + tid;
+            S.d.ltb[tid] = tid < 3u ? unkey_lo(S.pre[w]) : unkey_hi(S.pre[w]);
+            S.d.gtb[tid] = tid < 3u ? unkey_lo(S.bins[w]) : unkey_hi(S.bins[w]);
+        } else {
+            // kind 2: the forced median
+            S.d.kind = low == kNoKey ? (t.len > P.max_leaf ? 2u : 1u)
+                                     : (t.len <= P.max_leaf && __uint_as_float(low) >= leaf_cost(t.len) ? 1u : 0u);
+            S.d.axis = a;
+            S.d.split_bin = b;
+            S.d.n_lt = S.n_lt[a];
+            S.d.row = a * 32u + b;
+            S.d.use_thr = 0u;
+            S.d.thr = 0.0f;
+        }
+    }
+}
+
 // Stable partition of the large nodes' records into the other buffer: lt
 // records to the front of the node in order, gt records after them in order.
-// Each warp owns 256 consecutive records of the tile: a first pass computes
-// the side of each record (kept as 8 ballot words), one barrier publishes the
-// per-warp lt counts, and a second pass re-reads the records (cache hits) and
-// scatters them. Grid-stride over the level's tiles; also reduces the large
-// children's centroid bounds.
-constexpr uint32_t kPartPerLane = kTile / kTileThreads;  // 8
+// Each warp owns a run of consecutive records of the tile (at most
+// kPartPerLane times 32): a first pass computes the side of each record (kept
+// as ballot words; from the bin pass's codes, or against the threshold of a
+// learned split), one barrier publishes the per-warp lt counts, and a second
+// pass scatters the records. Grid-stride over the level's tiles; also reduces
+// the children's centroid bounds. kDecide: the CTA first decides its node's
+// split (part_decide), and the CTA of a node's first tile writes the node and
+// queues the children; otherwise an evaluation pass did (learned form, sample
+// output).
+constexpr uint32_t kPartPerLane = kTileMax / kTileThreads;
 
 #ifndef MGBVH_PART_MIN_BLOCKS
-#define MGBVH_PART_MIN_BLOCKS 5  // CTAs per SM the register budget must allow (tuning knob)
+// CTAs per SM the register budget must allow (tuning knob). Level passes at 3 /
+// 4 / 5 (80 / 64 / 48 registers, the last with spills): 0.581 / 0.537 / 0.556 ms
+// on the level-8 icosphere, 0.111 / 0.112 / 0.134 on 65,536 random triangles
+#define MGBVH_PART_MIN_BLOCKS 4
 #endif
 
+template <bool kDecide>
 __global__ void __launch_bounds__(kTileThreads, MGBVH_PART_MIN_BLOCKS) lvl_part_kernel(
-    const Task* __restrict__ tasks, const Decision* __restrict__ dec,
-    const uint32_t* __restrict__ tile_task, const uint32_t* __restrict__ tile_begin,
-    const uint32_t* __restrict__ tile_lt, Rec* rec0, Rec* rec1, const uint16_t* __restrict__ codes,
-    uint32_t* next_cbkeys, uint32_t lv, Out O) {
+    EvalArgs A, const TileRef* __restrict__ tiles, Rec* rec0, Rec* rec1, const uint16_t* __restrict__ codes,
+    uint32_t* next_cbkeys, Params P, Out O) {
     pdl_enter();
-    __shared__ uint32_t wcnt[kTileThreads / 32];
-    __shared__ uint32_t sk[12];
-    __shared__ int sbad;
-    const uint32_t ntiles = O.ctr->lvl[lv][1];
+    __shared__ PartSmem S;
+    const uint32_t ntiles = O.ctr->lvl[A.lv][1];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
+    uint32_t decided = 0xFFFFFFFFu;  // the node whose decision S.d holds
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t ti = tile_task[tile];
-        const Task& t = tasks[ti];
-        const Decision& d = dec[ti];
-        const uint32_t begin = tile_begin[tile];
-        const uint32_t tstart = t.start, tlen = t.len;
-        const uint32_t cnt = min(kTile, tlen - begin);
+        const TileRef tr = tiles[tile];
+        const uint32_t ti = tr.task, begin = tr.begin, cnt = tr.cnt;
+        const Task& t = A.tasks[ti];
+        const uint32_t tstart = t.start, tlen = t.len, cdepth = t.depth + 1u;
         const Rec* src = (t.buf ? rec1 : rec0) + tstart + begin;
         Rec* dst = t.buf ? rec0 : rec1;
-        if (d.kind == 1) {
-            for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
+        if (threadIdx.x < 12) S.keys[threadIdx.x] = ((threadIdx.x % 6) < 3) ? kKeyPosInf : kKeyNegInf;
+        if (threadIdx.x == 12) S.bad = 0;
+        if (threadIdx.x == 13) S.lt_off = 0;
+        if (ti == decided) {
+            // (a CTA's next tile often belongs to the same node)
+        } else if constexpr (kDecide) {
+            if (leaf_rule(tlen, t.depth, P)) {  // (the children queued are no leaves by the rule; a root may be)
+                if (threadIdx.x == 0) S.d.kind = 1u;
+            } else {
+                part_decide(S, A, t, ti, P);
+            }
+        } else {
+            if (threadIdx.x < sizeof(Decision) / 4u)
+                reinterpret_cast<uint32_t*>(&S.d)[threadIdx.x] = reinterpret_cast<const uint32_t*>(A.dec + ti)[threadIdx.x];
+        }
+        decided = ti;
+        __syncthreads();
+        const uint32_t kind = S.d.kind;
+        if (kind != 0u) {
+            for (uint32_t i = threadIdx.x; i < cnt; i += kTileThreads)
                 O.perm[tstart + begin + i] = __float_as_uint(src[i].lo.w);
+            if (kDecide && begin == 0u && warp == 0u) {
+                const Task tt = t;
+                if (kind == 1u)
+                    emit_leaf(P, O, lane, tt);
+                else if (lane == 0)
+                    queue_median(A, O, tt);
+            }
+            __syncthreads();
             continue;
         }
-        const uint32_t axis = d.axis, split_bin = d.split_bin, nbins = d.bins, n_lt = d.n_lt;
-        const float cmin = d.cmin, ext = d.ext, thr = d.thr;
-        const bool use_thr = d.use_thr != 0;
-        if (threadIdx.x < 12) sk[threadIdx.x] = ((threadIdx.x % 6) < 3) ? kKeyPosInf : kKeyNegInf;
-        if (threadIdx.x == 0) sbad = 0;
-        const uint32_t w0 = warp * (32u * kPartPerLane);
-        // pass 1: sides (from the bin pass's codes for a binned split; else the
-        // split axis's bounds of all this lane's records are loaded first)
+        const uint32_t axis = S.d.axis, split_bin = S.d.split_bin, n_lt = S.d.n_lt;
+        const bool use_thr = !kDecide && S.d.use_thr != 0;
+        {
+            // lt objects of the node's earlier tiles
+            const uint32_t* h = (use_thr ? A.tile_hist2 : A.tile_hist) + (size_t)S.d.row * A.cap_tiles + t.tile0;
+            uint32_t sum = 0;
+            for (uint32_t i = threadIdx.x; i < tile - t.tile0; i += kTileThreads) sum += h[i];
+            sum = __reduce_add_sync(kFull, sum);
+            if (lane == 0 && sum) atomicAdd(&S.lt_off, sum);
+        }
+        const uint32_t per = ((cnt + kTileThreads - 1u) / kTileThreads) * 32u, w0 = warp * per;
+        // pass 1: sides
         uint32_t bal[kPartPerLane];
         uint32_t lt_w = 0;
-        if (kPartCodes && !use_thr) {
-            // binned split: the bin pass left each record's bin on the split axis
+        if (!use_thr) {
             const uint16_t* cs = codes + tstart + begin;
             const uint32_t sh = 5u * axis;
             uint32_t cj[kPartPerLane];
 #pragma unroll
             for (uint32_t j = 0; j < kPartPerLane; ++j) {
                 const uint32_t i = w0 + j * 32u + lane;
-                cj[j] = i < cnt ? cs[i] : 0xFFFFu;
+                cj[j] = j * 32u < per && i < cnt ? cs[i] : 0xFFFFu;
             }
 #pragma unroll
             for (uint32_t j = 0; j < kPartPerLane; ++j) {
-                const bool pred = w0 + j * 32u + lane < cnt && ((cj[j] >> sh) & 31u) < split_bin;
+                const bool pred = j * 32u < per && w0 + j * 32u + lane < cnt && ((cj[j] >> sh) & 31u) < split_bin;
                 bal[j] = __ballot_sync(kFull, pred);
                 lt_w += __popc(bal[j]);
             }
         } else {
-            float pl[kPartPerLane], ph[kPartPerLane];
-#pragma unroll
-            for (uint32_t j = 0; j < kPartPerLane; ++j) {
-                const uint32_t i = w0 + j * 32u + lane;
-                if (i < cnt) {
-                    pl[j] = reinterpret_cast<const float*>(&src[i].lo)[axis];
-                    ph[j] = reinterpret_cast<const float*>(&src[i].hi)[axis];
-                }
-            }
+            const float thr = S.d.thr;
 #pragma unroll
             for (uint32_t j = 0; j < kPartPerLane; ++j) {
                 const uint32_t i = w0 + j * 32u + lane;
                 bool pred = false;
-                if (i < cnt) {
-                    const float c = center_of(pl[j], ph[j]);
-                    pred = use_thr ? c < thr : bin_of(c, cmin, ext, nbins) < split_bin;
-                }
+                if (j * 32u < per && i < cnt)
+                    pred = center_of(reinterpret_cast<const float*>(&src[i].lo)[axis],
+                                     reinterpret_cast<const float*>(&src[i].hi)[axis]) < thr;
                 bal[j] = __ballot_sync(kFull, pred);
                 lt_w += __popc(bal[j]);
             }
         }
-        if (lane == 0) wcnt[warp] = lt_w;
+        if (lane == 0) S.wcnt[warp] = lt_w;
         __syncthreads();
         uint32_t run = 0;
-        for (uint32_t q = 0; q < warp; ++q) run += wcnt[q];
-        const uint32_t lt_off = tile_lt[tile];
+        for (uint32_t q = 0; q < warp; ++q) run += S.wcnt[q];
+        const uint32_t lt_off = S.lt_off;
         const uint32_t lt_base = tstart + lt_off;
         const uint32_t gt_base = tstart + n_lt + (begin - lt_off);
-        const bool leaf_lt = d.child_leaf[1] != 0, leaf_gt = d.child_leaf[0] != 0;
-        uint32_t k[12];
-        init_key12(k);
-        bool bad = false;
+        const bool leaf_lt = leaf_rule(n_lt, cdepth, P), leaf_gt = leaf_rule(tlen - n_lt, cdepth, P);
+        SideBounds side;
+        uint32_t bad = 0;  // 1 a record outside its node's range or counts that differ, 2 a centroid outside
+        if (warp == kTileThreads / 32u - 1u && begin + cnt == tlen && lt_off + run + lt_w != n_lt) bad = 1u;
         // pass 2: scatter
 #pragma unroll(kPartUnroll)
         for (uint32_t j = 0; j < kPartPerLane; ++j) {
             const uint32_t i = w0 + j * 32u + lane;
+            if (j * 32u >= per) break;
             if (i < cnt) {
                 const Rec r = src[i];
                 const bool pred = (bal[j] >> lane) & 1u;
                 const uint32_t ltr = run + __popc(bal[j] & below);
                 const uint32_t dest = pred ? lt_base + ltr : gt_base + (i - ltr);
-                const float c0 = center_of(r.lo.x, r.hi.x), c1 = center_of(r.lo.y, r.hi.y),
-                            c2 = center_of(r.lo.z, r.hi.z);
                 if (dest - tstart < tlen) {
                     dst[dest] = r;
                     if (pred ? leaf_lt : leaf_gt) O.perm[dest] = __float_as_uint(r.lo.w);
                 } else {
-                    bad = true;  // inconsistent counts; never write outside the node
+                    bad = 1u;  // inconsistent counts; never write outside the node
                 }
-                bad |= !box_contains(pred ? d.ltb : d.gtb, c0, c1, c2);
-                const float c[3] = {c0, c1, c2};
-                grow_keys12(k, pred, c);
+                const float c[3] = {center_of(r.lo.x, r.hi.x), center_of(r.lo.y, r.hi.y), center_of(r.lo.z, r.hi.z)};
+                side.add(pred, c);
             }
             run += __popc(bal[j]);
         }
-        const bool need_lt = d.child_task[1] != kNone, need_gt = d.child_task[0] != kNone;
-        if (need_lt || need_gt) {
+        // containment of the centroids in their side's box (bvh/src/lib.rs:
+        // 637-646): the corners of the warp's centroid bounds on each side
+        const bool has_lt = __any_sync(kFull, side.lt[0] <= side.lt[3]), has_gt = __any_sync(kFull, side.gt[0] <= side.gt[3]);
+        float ck[12];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            ck[q] = q < 3 ? warp_min(side.lt[q]) : warp_max(side.lt[q]);
+            ck[6 + q] = q < 3 ? warp_min(side.gt[q]) : warp_max(side.gt[q]);
+        }
+        if (has_lt && !(box_contains(S.d.ltb, ck[0], ck[1], ck[2]) && box_contains(S.d.ltb, ck[3], ck[4], ck[5])))
+            bad |= 2u;
+        if (has_gt && !(box_contains(S.d.gtb, ck[6], ck[7], ck[8]) && box_contains(S.d.gtb, ck[9], ck[10], ck[11])))
+            bad |= 2u;
+        if (side.nan) bad |= 2u;
+        const bool need_lt = !leaf_lt && n_lt > P.medium_max, need_gt = !leaf_gt && tlen - n_lt > P.medium_max;
+        if ((need_lt || need_gt) && lane == 0) {
 #pragma unroll
             for (int q = 0; q < 12; ++q) {
-                const bool is_min = (q % 6) < 3;
-                const uint32_t v = is_min ? __reduce_min_sync(kFull, k[q]) : __reduce_max_sync(kFull, k[q]);
-                if (lane == 0) {
-                    if (is_min)
-                        atomicMin(&sk[q], v);
-                    else
-                        atomicMax(&sk[q], v);
-                }
-            }
-        }
-        if (__any_sync(kFull, bad) && lane == 0) sbad = 1;
-        __syncthreads();
-        if (threadIdx.x == 0 && sbad) set_error(O.ctr, MGBVH_ERR_ASSERT, kSiteContain);
-        if ((need_lt || need_gt) && threadIdx.x < 12) {
-            const uint32_t q = threadIdx.x;
-            const uint32_t child = q < 6 ? d.child_task[1] : d.child_task[0];
-            if (child != kNone) {
-                uint32_t* g = next_cbkeys + 6 * child + (q % 6);
                 if ((q % 6) < 3)
-                    atomicMin(g, sk[q]);
+                    atomicMin(&S.keys[q], fkey(ck[q]));
                 else
-                    atomicMax(g, sk[q]);
+                    atomicMax(&S.keys[q], fkey(ck[q]));
             }
         }
-        __syncthreads();  // wcnt/sk/sbad are rewritten by the next tile
+        if (bad) atomicOr(&S.bad, bad);
+        __syncthreads();
+        if (threadIdx.x == 0 && S.bad) set_error(O.ctr, MGBVH_ERR_ASSERT, S.bad & 1u ? kSiteCount : kSiteContain);
+        if (threadIdx.x < 12 && (threadIdx.x < 6 ? need_lt : need_gt)) {
+            uint32_t* g = next_cbkeys + 12 * ti + threadIdx.x;
+            if ((threadIdx.x % 6) < 3)
+                atomicMin(g, S.keys[threadIdx.x]);
+            else
+                atomicMax(g, S.keys[threadIdx.x]);
+        }
+        if (kDecide && begin == 0u && warp == 1u) {
+            const Task tt = t;
+            emit_split(A, P, O, ti, lane, tt, S.d);
+        }
+        __syncthreads();  // S is rewritten by the next tile
     }
 }
 
@@ -1386,8 +1483,8 @@ struct MedOut {
     Task* tasks;
     uint32_t* bins;
     uint32_t* cbkeys;
-    uint32_t* tile_task;
-    uint32_t* tile_begin;
+    TileRef* tiles;
+    uint32_t tile;  // most objects of a tile
     Task* medium;
     Task* small;
     uint32_t cap_tasks, cap_tiles, cap_medium, cap_small;
@@ -1625,11 +1722,11 @@ __global__ void __launch_bounds__(128) med_finish_kernel(const Task* __restrict_
             ct.pair = c == 0 ? t.pair + 2u : t.pair + 2u * (n - m);
             ct.depth = depth;
             ct.buf = t.buf ^ 1u;
-            ct.tile0 = ct.ntiles = 0;
+            ct.tile0 = ct.cb = 0;
             ct.nbase = t.nbase;
             ct.tbase = t.tbase;
             if (len > P.medium_max) {
-                const uint32_t nt = (len + kTile - 1) / kTile;
+                const uint32_t nt = tiles_of(len, M.tile);
                 uint32_t ti = 0, t0 = 0;
                 if (lane == 0) {
                     ti = atomicAdd(&O.ctr->lvl[0][0], 1u);
@@ -1642,14 +1739,11 @@ __global__ void __launch_bounds__(128) med_finish_kernel(const Task* __restrict_
                     continue;
                 }
                 ct.tile0 = t0;
-                ct.ntiles = nt;
+                ct.cb = ti;
                 if (lane == 0) M.tasks[ti] = ct;
                 init_task_bins(M.bins + (size_t)ti * kBinWords, lane, 32);
                 if (lane < 6) M.cbkeys[6 * ti + lane] = ck[(c == 0 ? 6 : 0) + lane];
-                for (uint32_t i = lane; i < nt; i += 32) {
-                    M.tile_task[t0 + i] = ti;
-                    M.tile_begin[t0 + i] = i * kTile;
-                }
+                write_tiles(M.tiles + t0, nt, ti, len, lane, 32);
             } else {
                 const bool med = len > kSmallMax;
                 uint32_t li = 0;
@@ -1758,25 +1852,6 @@ __device__ __forceinline__ void medium_leaf(const MS& S, uint32_t ib, uint32_t b
         if (depth == P.max_depth) atomicAdd(&O.ctr->depth_capped, 1u);
     }
 }
-
-// Centroid bounds of the lt and gt objects a lane has placed, and whether one
-// of them was NaN (which no bounds contain).
-struct SideBounds {
-    float lt[6], gt[6];  // min xyz, max xyz
-    bool nan;
-
-    __device__ __forceinline__ SideBounds() : nan(false) {
-        box_empty(lt);
-        box_empty(gt);
-    }
-    __device__ __forceinline__ void add(bool first, const float* c) {
-        nan |= c[0] != c[0] || c[1] != c[1] || c[2] != c[2];
-        if (first)
-            box_grow(lt, c[0], c[1], c[2], c[0], c[1], c[2]);
-        else
-            box_grow(gt, c[0], c[1], c[2], c[0], c[1], c[2]);
-    }
-};
 
 // Warp: stable partition of positions [p0, p1) of a node's list idx[ib] into
 // idx[ib ^ 1]: lt objects from position `lt_at` on, gt objects from `gt_at`
@@ -2243,7 +2318,7 @@ __device__ __forceinline__ void medium_task(MS& S, const Task t, Rec* rec0, Rec*
                     st.pair = pair;
                     st.depth = cdepth;
                     st.buf = t.buf;
-                    st.tile0 = st.ntiles = 0;
+                    st.tile0 = st.cb = 0;
                     st.nbase = t.nbase;
                     st.tbase = t.tbase;
                     small[si] = st;
@@ -2856,8 +2931,7 @@ __device__ __noinline__ void queue_large_task(const QueueArgs& Q, LargeSmem& L, 
         ltb[i] = L.ltb[i];
         gtb[i] = L.gtb[i];
     }
-    uint32_t k[12];
-    init_key12(k);
+    SideBounds side;
     bool bad = false;
     uint32_t run_lt = 0, run_gt = 0;
     constexpr uint32_t kPer = 4, kChunk = kMediumThreads * kPer;
@@ -2912,7 +2986,7 @@ __device__ __noinline__ void queue_large_task(const QueueArgs& Q, LargeSmem& L, 
                 const float c[3] = {center_of(r[g].lo.x, r[g].hi.x), center_of(r[g].lo.y, r[g].hi.y),
                                     center_of(r[g].lo.z, r[g].hi.z)};
                 bad |= !box_contains2(ltb, gtb, pred, c[0], c[1], c[2]);
-                grow_keys12(k, pred, c);
+                side.add(pred, c);
             }
             lt_run += __popc(bal[g]);
             gt_run += __popc(vm[g] & ~bal[g]);
@@ -2924,7 +2998,8 @@ __device__ __noinline__ void queue_large_task(const QueueArgs& Q, LargeSmem& L, 
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
         const bool is_min = (q % 6) < 3;
-        const uint32_t v = is_min ? __reduce_min_sync(kFull, k[q]) : __reduce_max_sync(kFull, k[q]);
+        const float b = q < 6 ? side.lt[q % 6] : side.gt[q % 6];
+        const uint32_t v = fkey(is_min ? warp_min(b) : warp_max(b));
         if (lane == 0) {
             if (is_min)
                 atomicMin(&L.keys[q], v);
@@ -2970,7 +3045,7 @@ __device__ __noinline__ void queue_large_task(const QueueArgs& Q, LargeSmem& L, 
             ct.pair = c == 0 ? t.pair + 2u : t.pair + 2u * n_gt;
             ct.depth = d1;
             ct.buf = t.buf ^ 1u;
-            ct.tile0 = ct.ntiles = 0;
+            ct.tile0 = ct.cb = 0;
             ct.nbase = t.nbase;
             ct.tbase = t.tbase;
             queue_push_main(Q, ct, len > P.medium_max ? L.keys + (c == 0 ? 6 : 0) : nullptr, O.ctr);
@@ -3226,7 +3301,7 @@ __global__ void init_mkeys_kernel(uint32_t* mkeys, uint32_t nm) {
 // One warp per mesh: queue its root (or finish it when the root is a leaf).
 __global__ void init_roots_kernel(const DevMesh* __restrict__ meshes, uint32_t nm,
                                   const uint32_t* __restrict__ mkeys, Task* large, uint32_t* bins,
-                                  uint32_t* cbkeys, uint32_t* tile_task, uint32_t* tile_begin,
+                                  uint32_t* cbkeys, TileRef* tiles,
                                   Task* medium, Task* small, Out O, uint32_t max_depth) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
@@ -3247,7 +3322,7 @@ __global__ void init_roots_kernel(const DevMesh* __restrict__ meshes, uint32_t n
         t.depth = 0;
         t.buf = 0;
         t.tile0 = M.tile0;
-        t.ntiles = M.ntiles;
+        t.cb = M.list_index;
         t.nbase = M.nbase;
         t.tbase = M.tbase;
         if (M.cls == 0) {
@@ -3265,10 +3340,7 @@ __global__ void init_roots_kernel(const DevMesh* __restrict__ meshes, uint32_t n
             if (lane == 0) large[M.list_index] = t;
             init_task_bins(bins + (size_t)M.list_index * kBinWords, lane, 32);
             if (lane < 6) cbkeys[6 * M.list_index + lane] = mkeys[12 * m + 6 + lane];
-            for (uint32_t i = lane; i < M.ntiles; i += 32) {
-                tile_task[M.tile0 + i] = M.list_index;
-                tile_begin[M.tile0 + i] = i * kTile;
-            }
+            write_tiles(tiles + M.tile0, M.ntiles, M.list_index, M.n, lane, 32);
         }
     }
 }
@@ -3306,7 +3378,7 @@ __global__ void queue_roots_kernel(const DevMesh* __restrict__ meshes, uint32_t 
         t.pair = 1;
         t.depth = 0;
         t.buf = 0;
-        t.tile0 = t.ntiles = 0;
+        t.tile0 = t.cb = 0;
         t.nbase = M.nbase;
         t.tbase = M.tbase;
         queue_push_main(Q, t, M.n > medium_max ? mkeys + 12 * m + 6 : nullptr, O.ctr);
@@ -3434,8 +3506,8 @@ struct mgbvh_ctx {
     cudaStream_t own = nullptr;     // the context's stream, kept for its life
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evp[3] = {nullptr, nullptr, nullptr};
     std::string err;
-    DevBuf rec[2], tasks[2], bins[2], cbkeys[2], tile_task[2], tile_begin[2];
-    DevBuf tile_hist, tile_lt, dec, medium, small, nodes, lens, used, newidx, widened, perm, ctr, cub_tmp;
+    DevBuf rec[2], tasks[2], bins[2], cbkeys[2], tiles[2];
+    DevBuf tile_hist, dec, medium, small, nodes, lens, used, newidx, widened, perm, ctr, cub_tmp;
     DevBuf bincode;  // per object of a level pass: its bin on each axis (5 bits each)
     DevBuf in_a, in_b, out_nodes, out_lens;
     DevBuf mesh_buf, toff_buf, noff_buf, mkeys;
@@ -3520,18 +3592,33 @@ T* P_(DevBuf& b) {
 
 struct Caps {
     uint32_t tasks, tiles, medium, small, nodes;
+    uint32_t tile;  // most objects of a level-pass tile
 };
+
+// Objects of a level-pass tile for a build of n objects. Up to one wave of
+// bin-pass CTAs (MGBVH_BIN_MIN_BLOCKS per SM), a tile for each, with a little
+// room for the ragged tiles of the lower levels; beyond, whole waves of tiles
+// near 2,048 objects. Less than 512 objects are not worth the merge of a
+// tile's bins (672 words).
+uint32_t tile_objects(uint32_t n, int sm_count) {
+    const uint64_t wave = (uint64_t)sm_count * MGBVH_BIN_MIN_BLOCKS * 31 / 32;
+    const uint64_t waves = std::max<uint64_t>(1, (n + wave * 1024) / (wave * 2048));
+    uint64_t tile = (n + wave * waves - 1) / (wave * waves);
+    if (tile > kTileMax) tile = (n + wave * (waves + 1) - 1) / (wave * (waves + 1));
+    return (uint32_t)std::min<uint64_t>(kTileMax, std::max<uint64_t>(512, (tile + 31) / 32 * 32));
+}
 
 // List capacities for n objects over `meshes` roots, each a bound that no
 // input can exceed: nodes above medium_max are disjoint at one level (<= n /
-// (medium_max + 1) of them, spanning <= n / kTile + that many tiles); the
+// (medium_max + 1) of them, spanning <= n / tile + that many tiles); the
 // queued subtrees of 33..medium_max objects are disjoint (none lies inside
 // another), so there are <= n / 33 of them, however unbalanced the tree; the
 // queued subtrees of 2..32 objects are disjoint too (<= n / 2).
-Caps caps_for(uint32_t n, uint32_t medium_max, uint32_t meshes, uint32_t node_slots) {
+Caps caps_for(uint32_t n, uint32_t medium_max, uint32_t meshes, uint32_t node_slots, int sm_count) {
     Caps c;
+    c.tile = tile_objects(n, sm_count);
     c.tasks = n / (medium_max + 1) + 2;
-    c.tiles = n / kTile + c.tasks + 2;
+    c.tiles = n / c.tile + c.tasks + 2;
     c.medium = n / (kSmallMax + 1) + meshes + 8;
     c.small = n / 2 + meshes + 8;
     c.nodes = node_slots;
@@ -3640,20 +3727,18 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
         for (uint32_t bl = 0; bl < batch; ++bl, ++level) {
             // buffers alternate between two sets; level counters rotate over three slots
             const uint32_t bf = level & 1u, nx = bf ^ 1u, lv = level % 3u;
-            launches += 3;
+            launches += 2;
             EvalArgs A;
             A.tasks = P_<Task>(ctx->tasks[bf]);
             A.lv = lv;
             A.bins = P_<uint32_t>(ctx->bins[bf]);
             A.cbkeys = P_<uint32_t>(ctx->cbkeys[bf]);
             A.tile_hist = P_<uint32_t>(ctx->tile_hist);
-            A.tile_lt = P_<uint32_t>(ctx->tile_lt);
             A.dec = P_<Decision>(ctx->dec);
             A.next_tasks = P_<Task>(ctx->tasks[nx]);
             A.next_bins = P_<uint32_t>(ctx->bins[nx]);
-            A.next_cbkeys = P_<uint32_t>(ctx->cbkeys[nx]);
-            A.next_tile_task = P_<uint32_t>(ctx->tile_task[nx]);
-            A.next_tile_begin = P_<uint32_t>(ctx->tile_begin[nx]);
+            A.next_tiles = P_<TileRef>(ctx->tiles[nx]);
+            A.tile = C.tile;
             A.medium = P_<Task>(ctx->medium);
             A.small = P_<Task>(ctx->small);
             A.cap_tasks = C.tasks;
@@ -3668,12 +3753,16 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
             A.rbins = LN.w ? P_<uint32_t>(ctx->rbins) : nullptr;
             A.tile_hist2 = LN.w ? P_<uint32_t>(ctx->tile_hist2) : nullptr;
             A.med = P_<Task>(ctx->med_list);
+            const TileRef* tiles = P_<TileRef>(ctx->tiles[bf]);
+            uint32_t* next_cbkeys = P_<uint32_t>(ctx->cbkeys[nx]);
             launch_k(lvl_bin_kernel, tile_grid, kTileThreads, 0, sm,
-                P_<Task>(ctx->tasks[bf]), P_<uint32_t>(ctx->cbkeys[bf]), P_<uint32_t>(ctx->bins[bf]),
-                P_<uint32_t>(ctx->tile_task[bf]), P_<uint32_t>(ctx->tile_begin[bf]),
+                A.tasks, A.cbkeys, next_cbkeys, P_<uint32_t>(ctx->bins[bf]), tiles,
                 P_<uint32_t>(ctx->tile_hist), C.tiles, rec0, rec1, P_<uint16_t>(ctx->bincode), d_ctr, lv, P);
-            launch_k(LN.w ? lvl_eval_kernel<true> : lvl_eval_kernel<false>, eval_grid, 128, LN.w ? kEvalWeightBytes : 0,
-                     sm, A, P, O);
+            const bool eval_pass = LN.w || LN.samples;
+            if (eval_pass) {
+                launch_k(lvl_eval_kernel, eval_grid, 128, LN.w ? kEvalWeightBytes : 0, sm, A, P, O);
+                launches++;
+            }
             if (LN.samples) {
                 launch_k(lvl_sample_kernel, ctx->sm_count * 2, 256, 0, sm,
                     A.tasks, A.dec, A.bins, A.cbkeys, rec0, rec1, d_ctr, lv, P, LN);
@@ -3681,16 +3770,13 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
             }
             if (LN.w) {
                 launch_k(lvl_refine_bin_kernel, tile_grid, kTileThreads, 0, sm,
-                    A.tasks, A.cbkeys, A.refine, A.rbins, P_<uint32_t>(ctx->tile_task[bf]),
-                    P_<uint32_t>(ctx->tile_begin[bf]), P_<uint32_t>(ctx->tile_hist2),
+                    A.tasks, A.cbkeys, A.refine, A.rbins, tiles, P_<uint32_t>(ctx->tile_hist2),
                     P_<uint32_t>(ctx->tile_hist), C.tiles, rec0, rec1, P_<uint16_t>(ctx->bincode), d_ctr, lv);
                 launch_k(lvl_eval2_kernel, eval_grid, 128, 0, sm, A, P, O);
                 launches += 2;
             }
-            launch_k(lvl_part_kernel, tile_grid, kTileThreads, 0, sm,
-                P_<Task>(ctx->tasks[bf]), P_<Decision>(ctx->dec), P_<uint32_t>(ctx->tile_task[bf]),
-                P_<uint32_t>(ctx->tile_begin[bf]), P_<uint32_t>(ctx->tile_lt), rec0, rec1,
-                P_<uint16_t>(ctx->bincode), P_<uint32_t>(ctx->cbkeys[nx]), lv, O);
+            launch_k(eval_pass ? lvl_part_kernel<false> : lvl_part_kernel<true>, tile_grid, kTileThreads, 0, sm,
+                A, tiles, rec0, rec1, P_<uint16_t>(ctx->bincode), next_cbkeys, P, O);
         }
         MG_CUDA(cudaGetLastError());
         if (fixed_levels || optimistic) break;
@@ -3875,8 +3961,8 @@ int run_medians(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, Re
         M.tasks = P_<Task>(ctx->tasks[0]);
         M.bins = P_<uint32_t>(ctx->bins[0]);
         M.cbkeys = P_<uint32_t>(ctx->cbkeys[0]);
-        M.tile_task = P_<uint32_t>(ctx->tile_task[0]);
-        M.tile_begin = P_<uint32_t>(ctx->tile_begin[0]);
+        M.tiles = P_<TileRef>(ctx->tiles[0]);
+        M.tile = C.tile;
         M.medium = P_<Task>(ctx->medium);
         M.small = P_<Task>(ctx->small);
         M.cap_tasks = C.tasks;
@@ -3907,7 +3993,7 @@ int run_build(mgbvh_ctx* ctx, const Input& in, const mgbvh_settings* st, mgbvh_n
     const uint32_t n = in.n;
     const cudaStream_t sm = ctx->stream;
     if (n > 0x7FFFFFFFu) return fail(ctx, MGBVH_ERR_UNSUPPORTED, "more than 2^31-1 objects");
-    const Caps C = caps_for(n, ctx->medium_max, 1, 2 * n - 1);
+    const Caps C = caps_for(n, ctx->medium_max, 1, 2 * n - 1, ctx->sm_count);
     int rc;
 #define ENS(buf, bytes) \
     if ((rc = ensure(ctx, buf, (bytes))) != MGBVH_OK) return rc
@@ -3916,12 +4002,10 @@ int run_build(mgbvh_ctx* ctx, const Input& in, const mgbvh_settings* st, mgbvh_n
     for (int i = 0; i < 2; ++i) {
         ENS(ctx->tasks[i], sizeof(Task) * (size_t)C.tasks);
         ENS(ctx->bins[i], 4ull * kBinWords * C.tasks);
-        ENS(ctx->cbkeys[i], 24ull * C.tasks);
-        ENS(ctx->tile_task[i], 4ull * C.tiles);
-        ENS(ctx->tile_begin[i], 4ull * C.tiles);
+        ENS(ctx->cbkeys[i], 48ull * C.tasks);  // both children of a node
+        ENS(ctx->tiles[i], sizeof(TileRef) * (size_t)C.tiles);
     }
     ENS(ctx->tile_hist, 4ull * 96 * C.tiles);  // [axis][bin][tile]
-    ENS(ctx->tile_lt, 4ull * C.tiles);
     ENS(ctx->bincode, 2ull * n);
     ENS(ctx->dec, sizeof(Decision) * (size_t)C.tasks);
     ENS(ctx->med_list, sizeof(Task) * (size_t)C.tasks);
@@ -3984,20 +4068,19 @@ int run_build(mgbvh_ctx* ctx, const Input& in, const mgbvh_settings* st, mgbvh_n
         if ((rc = ensure(ctx, ctx->medium2, sizeof(Task) * (size_t)C.medium)) != MGBVH_OK) return rc;
         ctx->stream_slots = C.nodes;
     }
-    const uint32_t ntiles0 = (n + kTile - 1) / kTile;
+    const uint32_t ntiles0 = tiles_of(n, C.tile);
     const float* bb = st->bounds;
     {
         const int blocks = (int)std::min<uint32_t>((std::max(n, ntiles0) + 255) / 256 + 1, 1024u);
         launch_k(init_root_kernel, blocks, 256, 0, sm,
             n, cls, st->has_bounds, bb[0], bb[1], bb[2], bb[3], bb[4], bb[5], P_<Task>(ctx->tasks[0]),
-            P_<uint32_t>(ctx->bins[0]), P_<uint32_t>(ctx->cbkeys[0]), P_<uint32_t>(ctx->tile_task[0]),
-            P_<uint32_t>(ctx->tile_begin[0]), P_<Task>(ctx->medium), P_<Task>(ctx->small), O, ntiles0,
+            P_<uint32_t>(ctx->bins[0]), P_<uint32_t>(ctx->cbkeys[0]), P_<TileRef>(ctx->tiles[0]),
+            P_<Task>(ctx->medium), P_<Task>(ctx->small), O, ntiles0,
             st->max_depth);
     }
     MG_CUDA(cudaGetLastError());
     MG_CUDA(cudaEventRecord(ctx->evp[0], sm));
     uint32_t launches = 2, levels = 0;
-    (void)ntiles0;
 
     const bool optimistic = cls == 3 && ctx->levels_hint > 0;
     if ((rc = run_pipeline(ctx, C, P, O, rec0, rec1, n, cls == 3, 0, launches, levels, optimistic)) != MGBVH_OK)
@@ -4149,6 +4232,9 @@ struct BatchPlan {
 
 int plan_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const mgbvh_settings* st,
                BatchPlan& B) {
+    uint64_t objects = 0;
+    for (uint32_t m = 0; m < nm; ++m) objects += meshes[m].count;
+    const uint32_t tile = tile_objects((uint32_t)std::min<uint64_t>(objects, 0x7FFFFFFFull), ctx->sm_count);
     B.nm = nm;
     B.hm.assign(nm, DevMesh());
     B.toffs.assign(nm + 1, 0);
@@ -4198,7 +4284,7 @@ int plan_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const
             M.cls = 3;
             M.list_index = B.n_large++;
             M.tile0 = B.tiles;
-            M.ntiles = (n + kTile - 1) / kTile;
+            M.ntiles = tiles_of(n, tile);
             B.tiles += M.ntiles;
         }
     }
@@ -4312,7 +4398,7 @@ int enqueue_batch(mgbvh_ctx* ctx, const BatchPlan& B, const Caps& C, const mgbvh
     } else {
         init_roots_kernel<<<std::max(1u, std::min((nm + 7) / 8, 1024u)), 256, 0, sm>>>(
             dmesh, nm, P_<uint32_t>(ctx->mkeys), P_<Task>(ctx->tasks[0]), P_<uint32_t>(ctx->bins[0]),
-            P_<uint32_t>(ctx->cbkeys[0]), P_<uint32_t>(ctx->tile_task[0]), P_<uint32_t>(ctx->tile_begin[0]),
+            P_<uint32_t>(ctx->cbkeys[0]), P_<TileRef>(ctx->tiles[0]),
             P_<Task>(ctx->medium), P_<Task>(ctx->small), O, st->max_depth);
         MG_CUDA(cudaGetLastError());
         if (!fixed_levels) MG_CUDA(cudaEventRecord(ctx->evp[0], sm));
@@ -4348,7 +4434,7 @@ int run_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const 
         return MGBVH_WARN_EMPTY;
     }
     const uint32_t n = B.n;
-    const Caps C = caps_for(n, ctx->medium_max, nm, B.slots);
+    const Caps C = caps_for(n, ctx->medium_max, nm, B.slots, ctx->sm_count);
 #define ENS(buf, bytes) \
     if ((rc = ensure(ctx, buf, (bytes))) != MGBVH_OK) return rc
     ENS(ctx->rec[0], sizeof(Rec) * (size_t)n);
@@ -4356,12 +4442,10 @@ int run_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const 
     for (int i = 0; i < 2; ++i) {
         ENS(ctx->tasks[i], sizeof(Task) * (size_t)C.tasks);
         ENS(ctx->bins[i], 4ull * kBinWords * C.tasks);
-        ENS(ctx->cbkeys[i], 24ull * C.tasks);
-        ENS(ctx->tile_task[i], 4ull * C.tiles);
-        ENS(ctx->tile_begin[i], 4ull * C.tiles);
+        ENS(ctx->cbkeys[i], 48ull * C.tasks);  // both children of a node
+        ENS(ctx->tiles[i], sizeof(TileRef) * (size_t)C.tiles);
     }
     ENS(ctx->tile_hist, 4ull * 96 * C.tiles);
-    ENS(ctx->tile_lt, 4ull * C.tiles);
     ENS(ctx->bincode, 2ull * n);
     ENS(ctx->dec, sizeof(Decision) * (size_t)C.tasks);
     ENS(ctx->med_list, sizeof(Task) * (size_t)C.tasks);
@@ -4805,9 +4889,8 @@ void mgbvh_destroy(mgbvh_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     DevBuf* all[] = {&ctx->rec[0], &ctx->rec[1], &ctx->tasks[0], &ctx->tasks[1], &ctx->bins[0],
-                     &ctx->bins[1], &ctx->cbkeys[0], &ctx->cbkeys[1], &ctx->tile_task[0],
-                     &ctx->tile_task[1], &ctx->tile_begin[0], &ctx->tile_begin[1], &ctx->tile_hist,
-                     &ctx->tile_lt, &ctx->dec, &ctx->medium, &ctx->small, &ctx->nodes, &ctx->lens,
+                     &ctx->bins[1], &ctx->cbkeys[0], &ctx->cbkeys[1], &ctx->tiles[0],
+                     &ctx->tiles[1], &ctx->tile_hist, &ctx->dec, &ctx->medium, &ctx->small, &ctx->nodes, &ctx->lens,
                      &ctx->used, &ctx->newidx, &ctx->widened, &ctx->perm, &ctx->ctr, &ctx->cub_tmp, &ctx->in_a,
                      &ctx->in_b, &ctx->out_nodes, &ctx->out_lens, &ctx->mesh_buf,
                      &ctx->toff_buf, &ctx->noff_buf, &ctx->mkeys, &ctx->learn_wt, &ctx->lref,
@@ -5169,7 +5252,7 @@ int mgbvh_build_aabbs_noalloc(const float* d_aabbs, uint32_t count, const mgbvh_
     const float* bb = st->bounds;
     init_root_kernel<<<(n + 255) / 256, 256, 0, sm>>>(n, cls, st->has_bounds, bb[0], bb[1], bb[2],
                                                       bb[3], bb[4], bb[5], nullptr, nullptr, nullptr,
-                                                      nullptr, nullptr, S->medium, S->small, O, 0u,
+                                                      nullptr, S->medium, S->small, O, 0u,
                                                       st->max_depth);
     if (cls == 2)
         medium_kernel<false, kMediumMax, kWidestWarps>

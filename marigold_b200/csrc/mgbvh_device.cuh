@@ -183,6 +183,10 @@ __device__ __forceinline__ uint64_t cand_key(float cost, uint32_t axis, uint32_t
     return (static_cast<uint64_t>(fkey(cost)) << 32) | (axis << 8) | idx;
 }
 
+__device__ __forceinline__ bool leaf_rule(uint32_t n, uint32_t depth, const Params& P) {
+    return n <= 1u || depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf);  // bvh/src/lib.rs:548, 556
+}
+
 // Minimum and maximum over the warp (one instruction on sm_100a).
 __device__ __forceinline__ float warp_min(float v) {
     float r;
@@ -324,6 +328,25 @@ __device__ __forceinline__ void shfl_cand(Cand& c, uint32_t src) {
     }
 }
 
+// Centroid bounds of the lt and gt objects a lane has placed, and whether one
+// of them was NaN (which no bounds contain).
+struct SideBounds {
+    float lt[6], gt[6];  // min xyz, max xyz
+    bool nan;
+
+    __device__ __forceinline__ SideBounds() : nan(false) {
+        box_empty(lt);
+        box_empty(gt);
+    }
+    __device__ __forceinline__ void add(bool first, const float* c) {
+        nan |= c[0] != c[0] || c[1] != c[1] || c[2] != c[2];
+        if (first)
+            box_grow(lt, c[0], c[1], c[2], c[0], c[1], c[2]);
+        else
+            box_grow(gt, c[0], c[1], c[2], c[0], c[1], c[2]);
+    }
+};
+
 // Bin index of a centroid on one axis of a node, as bin_of gives it. Instead of
 // the divide, the centroid is scaled by bins / ext; the exact form runs only
 // where the scaled value lies within 2^-14 of an integer (the two differ by
@@ -389,8 +412,12 @@ __device__ __forceinline__ void clear_bins(uint32_t* wb, uint32_t tid, uint32_t 
     for (uint32_t w = tid; w < kSweepWords; w += nthreads) wb[w] = 0u;
 }
 
-// Adds an object to its bins; returns the bins (5 bits per axis).
-__device__ __forceinline__ uint32_t add_to_bins(uint32_t* wb, const BinMap* map, const float4& lo, const float4& hi) {
+// Adds an object to its bins; returns the bins (5 bits per axis). On the axes in
+// `dense` a box key goes to its bin only where it extends the bin as read
+// before: lanes that share a bin read it at once, while their atomics on one
+// word take turns.
+__device__ __forceinline__ uint32_t add_to_bins(uint32_t* wb, const BinMap* map, const float4& lo, const float4& hi,
+                                                uint32_t dense = 0) {
     const uint32_t k[6] = {key_lo(lo.x), key_lo(lo.y), key_lo(lo.z), key_hi(hi.x), key_hi(hi.y), key_hi(hi.z)};
     const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
     uint32_t code = 0;
@@ -401,10 +428,34 @@ __device__ __forceinline__ uint32_t add_to_bins(uint32_t* wb, const BinMap* map,
         code |= b << (5u * a);
         uint32_t* w = wb + a * kSweepAxis + b * 7u;
         atomicAdd(w, 1u);
+        if ((dense >> a) & 1u) {
+            bool more[6];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) atomicMax(w + 1 + i, k[i]);
+            for (int i = 0; i < 6; ++i) more[i] = k[i] > *reinterpret_cast<volatile uint32_t*>(w + 1 + i);
+#pragma unroll
+            for (int i = 0; i < 6; ++i)
+                if (more[i]) atomicMax(w + 1 + i, k[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) atomicMax(w + 1 + i, k[i]);
+        }
     }
     return code;
+}
+
+// The axes (bits 0..2) on which at least kDenseLanes lanes' objects fall in
+// lane 0's bin. All lanes take part; lane 0 has an object.
+constexpr uint32_t kDenseLanes = 8;
+__device__ __forceinline__ uint32_t shared_bins(const BinMap* map, const float4& lo, const float4& hi, bool valid) {
+    const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+    uint32_t dense = 0;
+#pragma unroll
+    for (uint32_t a = 0; a < 3; ++a) {
+        const uint32_t b = valid ? map[a](l[a], h[a]) : kMaxBins;
+        const uint32_t same = __ballot_sync(kFull, b == __shfl_sync(kFull, b, 0));
+        dense |= __popc(same) >= kDenseLanes ? 1u << a : 0u;
+    }
+    return dense;
 }
 
 struct SweepResult {
@@ -612,10 +663,6 @@ __device__ __forceinline__ int top_bit(uint32_t m) {
     int r;
     asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(m));
     return r;
-}
-
-__device__ __forceinline__ bool leaf_rule(uint32_t n, uint32_t depth, const Params& P) {
-    return n <= 1u || depth == P.max_depth || (n <= P.max_leaf && n < 2u * P.min_leaf);  // bvh/src/lib.rs:548, 556
 }
 
 // Split profiles other than the reference's own (every node of <= 32 objects
