@@ -772,7 +772,7 @@ def run_batched(args):
                                           "meets, every triangle of its mesh"},
                   "rays_from": "origins uniform in the instances' world box grown by 10%, uniform directions",
                   "traversal": "two-level: TLAS with the world ray, each instance's BLAS in mesh space "
-                               "(scene.slang:91-220); one thread per ray, rays sorted"},
+                               "(scene.slang:91-220); persistent warps, rays sorted"},
         "value": round(total / (ms * 1e-3) / 1e6, 2), "unit": "Mtri/s", "ms_per_step": round(ms, 3),
         "clocks": clocks_best, "batch_mode": best, "modes": modes,
         "eager_first_build_ms": round(eager_ms, 3), "graph_replays": replays, "steps": args.steps,
