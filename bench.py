@@ -42,12 +42,12 @@ UNIT = "Mtri/s"
 SAMPLE_TRIS = 131072
 # dram__bytes_read.sum + dram__bytes_write.sum of one small_kernel launch on
 # this workload (24 warps per SM), from an ncu capture (cold cache):
-# 52.85 MB + 58.80 MB
-SMALL_KERNEL_TRAFFIC = 111650048
+# 46.58 MB + 50.57 MB
+SMALL_KERNEL_TRAFFIC = 97153536
 # smsp__inst_executed.sum of the same launch (warp instructions, spill loads
 # and stores included); the issue ceiling is one warp instruction per SM
 # sub-partition per cycle
-SMALL_KERNEL_INST = 464942099
+SMALL_KERNEL_INST = 320964808
 SM_SUBPARTITIONS = 4
 WORKLOAD = ("noisy icosphere L8 (1,310,720 tris, 655,362 verts), leaf 1, max_depth 32, "
             "reference split profile")
@@ -480,7 +480,7 @@ def run_ours(args):
                      "algorithmic_bytes_per_launch": int(small_alg),
                      "launch_ms": round(small_ms, 4), "subtrees": small_tasks,
                      "issue": issue_roofline(SMALL_KERNEL_INST, small_ms, clocks.summary()),
-                     "note": "issue-bound: the adaptive sweep's O(n^2) threshold evaluation"},
+                     "note": "issue-bound: mask and shuffle reads of every threshold's two boxes"},
         "roofline_build": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm,
                            "unit": "GB/s", "frac": round(achieved / hbm, 4),
                            "algorithmic_bytes_per_build": int(alg), "inner_len_sum": S},
