@@ -139,7 +139,10 @@ MGBVH_API void mgbvh_default_settings(mgbvh_settings* s);
 /* Device context: owns scratch buffers (grown on demand), a stream and events. */
 MGBVH_API int mgbvh_create(int device, mgbvh_ctx** out_ctx);
 MGBVH_API void mgbvh_destroy(mgbvh_ctx* ctx);
-/* Run subsequent builds on a caller stream (cudaStream_t); NULL = own stream. */
+/* Run subsequent builds on a caller stream (cudaStream_t); NULL = own stream,
+   which is ordered after no other (the caller's device arrays must be ready);
+   cudaStreamLegacy = own stream, and every call on device arrays first waits
+   for the work that is in the legacy default stream. */
 MGBVH_API int mgbvh_set_stream(mgbvh_ctx* ctx, void* cuda_stream);
 /* Text of the last error recorded on this context. */
 MGBVH_API const char* mgbvh_last_error(const mgbvh_ctx* ctx);

@@ -24,6 +24,7 @@ ERR_UNSUPPORTED = -6
 ERR_NO_DEVICE = -7
 ERR_TOO_LARGE = -8
 NOALLOC_MAX_OBJECTS = 1024
+STREAM_LEGACY = 1  # cudaStreamLegacy: the legacy default stream by name
 
 # every entry point declared in include/mgbvh.h
 EXPORTED = (
@@ -227,7 +228,9 @@ def status_string(status: int) -> str:
 
 
 class Context:
-    """An mgbvh_ctx: one CUDA device, its stream and scratch buffers."""
+    """An mgbvh_ctx: one CUDA device, its stream and scratch buffers. Calls on
+    device tensors run after the work in the default stream until set_stream
+    names another one."""
 
     def __init__(self, device: int = 0):
         self.L = load()
@@ -235,6 +238,7 @@ class Context:
         rc = self.L.mgbvh_create(device, ctypes.byref(self.ptr))
         if rc != OK:
             raise MgbvhError(rc, status_string(rc))
+        self.set_stream(0)
 
     def last_error(self) -> str:
         return self.L.mgbvh_last_error(self.ptr).decode()
@@ -245,7 +249,12 @@ class Context:
         return rc
 
     def set_stream(self, stream_handle: int | None):
-        self.check(self.L.mgbvh_set_stream(self.ptr, ctypes.c_void_p(stream_handle or 0)))
+        """A stream by its handle, as torch gives it: 0 is the default stream
+        (calls on device tensors wait for what is in it). None: the context's
+        own stream, ordered after no other."""
+        if stream_handle == 0:
+            stream_handle = STREAM_LEGACY
+        self.check(self.L.mgbvh_set_stream(self.ptr, ctypes.c_void_p(stream_handle)))
 
     def set_tuning(self, medium_max: int):
         self.check(self.L.mgbvh_set_tuning(self.ptr, medium_max))

@@ -3504,6 +3504,8 @@ struct mgbvh_ctx {
     uint32_t medium_max = kMediumMax;  // level-pass / subtree switch-over (speed only)
     cudaStream_t stream = nullptr;  // builds run here: own, or the caller's
     cudaStream_t own = nullptr;     // the context's stream, kept for its life
+    bool after_default = false;     // calls on device arrays wait for the legacy default stream first
+    cudaEvent_t evd = nullptr;      // ... through this event
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evp[3] = {nullptr, nullptr, nullptr};
     std::string err;
     DevBuf rec[2], tasks[2], bins[2], cbkeys[2], tiles[2];
@@ -4648,7 +4650,7 @@ int run_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const 
         cudaGraph_t g = nullptr;
         uint32_t gl = 0, glev = 0;
         const uint32_t fixed = (B.n_large > 0 ? levels : 0) + 1;
-        // (capture is not possible on the legacy default stream: then no graph)
+        // (a stream that cannot be captured, or is being captured already: then no graph)
         if (cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
         } else {
@@ -4702,6 +4704,17 @@ int check_ctx(mgbvh_ctx* ctx) {
     return MGBVH_OK;
 }
 
+// Orders the context's stream after the work in the legacy default stream
+// (mgbvh_set_stream with cudaStreamLegacy), for a call that reads or writes the
+// caller's device arrays. The other direction needs nothing: such calls return
+// when their work is done.
+int order_after_default(mgbvh_ctx* ctx) {
+    if (!ctx->after_default) return MGBVH_OK;
+    MG_CUDA(cudaEventRecord(ctx->evd, cudaStreamLegacy));
+    MG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->evd, 0));
+    return MGBVH_OK;
+}
+
 int build_common(mgbvh_ctx* ctx, const Input& in_dev, const mgbvh_settings* s, mgbvh_node* d_nodes,
                  uint32_t cap, uint32_t* out_count, uint32_t* d_lens, uint32_t* d_perm,
                  mgbvh_stats* stats) {
@@ -4715,6 +4728,7 @@ int build_common(mgbvh_ctx* ctx, const Input& in_dev, const mgbvh_settings* s, m
         return MGBVH_WARN_EMPTY;
     }
     if (!d_nodes || !d_perm) return fail(ctx, MGBVH_ERR_INVALID_ARG, "output pointer is NULL");
+    if ((rc = order_after_default(ctx)) != MGBVH_OK) return rc;
     return run_build(ctx, in_dev, s, d_nodes, cap, d_lens, d_perm, out_count, stats);
 }
 
@@ -4742,6 +4756,8 @@ int build_host(mgbvh_ctx* ctx, Input in, const mgbvh_settings* s, mgbvh_node* ou
         return MGBVH_WARN_EMPTY;
     }
     if (!out_nodes || !out_perm) return fail(ctx, MGBVH_ERR_INVALID_ARG, "output pointer is NULL");
+    // (the sample buffer is the only device array of the caller's here)
+    if (ctx->learn_samples && (rc = order_after_default(ctx)) != MGBVH_OK) return rc;
     const cudaStream_t sm = ctx->stream;
     Input d = in;
     if (in.kind == kIndexed) {
@@ -4872,6 +4888,7 @@ int mgbvh_create(int device, mgbvh_ctx** out_ctx) {
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
         cudaEventCreate(&ctx->evp[0]) != cudaSuccess || cudaEventCreate(&ctx->evp[1]) != cudaSuccess ||
         cudaEventCreate(&ctx->evp[2]) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->evd, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&ctx->h_ctr, sizeof(Counters)) != cudaSuccess ||
         cudaMallocHost(&ctx->h_init, sizeof(Counters)) != cudaSuccess ||
         !medium_smem_limits()) {
@@ -4912,6 +4929,7 @@ void mgbvh_destroy(mgbvh_ctx* ctx) {
     if (ctx->medium2.p) cudaFree(ctx->medium2.p);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    if (ctx->evd) cudaEventDestroy(ctx->evd);
     for (cudaEvent_t e : ctx->evp)
         if (e) cudaEventDestroy(e);
     if (ctx->own) cudaStreamDestroy(ctx->own);
@@ -4920,9 +4938,13 @@ void mgbvh_destroy(mgbvh_ctx* ctx) {
 
 int mgbvh_set_stream(mgbvh_ctx* ctx, void* stream) {
     if (!ctx) return MGBVH_ERR_INVALID_ARG;
-    // a caller that names no stream before each build (torch's default stream
-    // is handle 0) goes back to the same one: a new stream took 0.109 ms a call
-    ctx->stream = stream ? reinterpret_cast<cudaStream_t>(stream) : ctx->own;
+    // The own stream is kept for a caller that names no stream before each build:
+    // a new one took 0.109 ms a call. The legacy default stream is not built on
+    // but waited for (order_after_default): it cannot be captured into a graph,
+    // and builds of several contexts would take turns on it.
+    const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    ctx->after_default = s == cudaStreamLegacy;
+    ctx->stream = s && !ctx->after_default ? s : ctx->own;
     return MGBVH_OK;
 }
 
@@ -5000,6 +5022,7 @@ int mgbvh_build_batch_dev(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_
     if ((mesh_count && !meshes) || !out_node_offsets)
         return fail(ctx, MGBVH_ERR_INVALID_ARG, "meshes / out_node_offsets is NULL");
     if (!d_out_nodes || !d_out_perm) return fail(ctx, MGBVH_ERR_INVALID_ARG, "output pointer is NULL");
+    if ((rc = order_after_default(ctx)) != MGBVH_OK) return rc;
     return run_batch(ctx, meshes, mesh_count, settings, d_out_nodes, node_capacity, d_out_lens,
                      d_out_perm, out_node_offsets, out_stats);
 }
@@ -5015,6 +5038,7 @@ int mgbvh_set_split_proposer(mgbvh_ctx* ctx, const void* d_weights_bf16, int gat
     ctx->learn_gate = gate != 0;
     if (!d_weights_bf16) return MGBVH_OK;
     if (int rc = ensure(ctx, ctx->learn_wt, sizeof(__nv_bfloat16) * mgbvh_mlp::kTParams)) return rc;
+    if (int rc = order_after_default(ctx)) return rc;
     transpose_weights_kernel<<<(mgbvh_mlp::kTParams + 255) / 256, 256, 0, ctx->stream>>>(
         static_cast<const __nv_bfloat16*>(d_weights_bf16), P_<__nv_bfloat16>(ctx->learn_wt));
     MG_CUDA(cudaGetLastError());
@@ -5140,6 +5164,7 @@ int mgbvh_instance_aabbs_dev(mgbvh_ctx* ctx, const float* d_mesh_bounds, uint32_
     if (!d_mesh_bounds || !d_instance_mesh || !d_transforms || !d_out_aabbs)
         return fail(ctx, MGBVH_ERR_INVALID_ARG, "a device pointer is NULL");
     if ((rc = ensure(ctx, ctx->ctr, sizeof(Counters))) != MGBVH_OK) return rc;
+    if ((rc = order_after_default(ctx)) != MGBVH_OK) return rc;
     const cudaStream_t sm = ctx->stream;
     Counters* d_ctr = P_<Counters>(ctx->ctr);
     MG_CUDA(cudaMemsetAsync(d_ctr, 0, 2 * sizeof(uint32_t), sm));  // error, error_site
