@@ -3575,10 +3575,23 @@ int fail(mgbvh_ctx* ctx, int status, const std::string& msg) {
                         std::string(#call) + ": " + cudaGetErrorString(e_));               \
     } while (0)
 
+// Forgets the captured graph of batched builds.
+void drop_graph(mgbvh_ctx* ctx) {
+    if (!ctx->graph_exec) return;
+    cudaGraphExecDestroy(ctx->graph_exec);
+    ctx->graph_exec = nullptr;
+    ctx->graph_sig.clear();
+}
+
+// A scratch buffer of at least `bytes`. Any build may grow one, so a captured
+// graph, which holds the old address, goes with it.
 int ensure(mgbvh_ctx* ctx, DevBuf& b, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (b.bytes >= bytes) return MGBVH_OK;
-    if (b.p) cudaFree(b.p);
+    if (b.p) {
+        drop_graph(ctx);
+        cudaFree(b.p);
+    }
     b.p = nullptr;
     b.bytes = 0;
     const size_t want = bytes + bytes / 8;
@@ -4489,12 +4502,7 @@ int run_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const 
     // pinned staging of the plan
     const size_t pin_bytes = sizeof(Counters) + sizeof(DevMesh) * (size_t)nm + 8ull * (nm + 1);
     if (ctx->pin_bytes < pin_bytes) {
-        // a graph captured against the old staging must not be replayed
-        if (ctx->graph_exec) {
-            cudaGraphExecDestroy(ctx->graph_exec);
-            ctx->graph_exec = nullptr;
-            ctx->graph_sig.clear();
-        }
+        drop_graph(ctx);  // captured against the old staging
         if (ctx->pin) cudaFreeHost(ctx->pin);
         ctx->pin = nullptr;
         ctx->pin_bytes = 0;
@@ -4642,11 +4650,7 @@ int run_batch(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_t nm, const 
     MG_CUDA(cudaStreamSynchronize(sm));
     // capture a graph for the next build of this mesh set
     if (ctx->graph_mode && !from_graph && !had_medians && hc.holes == 0 && cap >= B.slots) {
-        if (ctx->graph_exec) {
-            cudaGraphExecDestroy(ctx->graph_exec);
-            ctx->graph_exec = nullptr;
-        }
-        ctx->graph_sig.clear();
+        drop_graph(ctx);
         cudaGraph_t g = nullptr;
         uint32_t gl = 0, glev = 0;
         const uint32_t fixed = (B.n_large > 0 ? levels : 0) + 1;
@@ -5029,11 +5033,7 @@ int mgbvh_build_batch_dev(mgbvh_ctx* ctx, const mgbvh_mesh_desc* meshes, uint32_
 
 int mgbvh_set_split_proposer(mgbvh_ctx* ctx, const void* d_weights_bf16, int gate) {
     if (int rc = check_ctx(ctx)) return rc;
-    if (ctx->graph_exec) {  // a captured graph holds the old switch
-        cudaGraphExecDestroy(ctx->graph_exec);
-        ctx->graph_exec = nullptr;
-        ctx->graph_sig.clear();
-    }
+    drop_graph(ctx);  // it holds the old switch
     ctx->learn_w = nullptr;
     ctx->learn_gate = gate != 0;
     if (!d_weights_bf16) return MGBVH_OK;
@@ -5050,11 +5050,7 @@ int mgbvh_set_split_proposer(mgbvh_ctx* ctx, const void* d_weights_bf16, int gat
 int mgbvh_set_proposer_gate(mgbvh_ctx* ctx, float refine_threshold, uint32_t min_objects) {
     if (!ctx) return MGBVH_ERR_INVALID_ARG;
     if (!(refine_threshold == refine_threshold)) return fail(ctx, MGBVH_ERR_INVALID_ARG, "refine_threshold is NaN");
-    if (ctx->graph_exec) {  // a captured graph holds the old gate
-        cudaGraphExecDestroy(ctx->graph_exec);
-        ctx->graph_exec = nullptr;
-        ctx->graph_sig.clear();
-    }
+    drop_graph(ctx);  // it holds the old gate
     ctx->learn_gate_thr = refine_threshold;
     ctx->learn_min_n = min_objects;
     return MGBVH_OK;
@@ -5067,9 +5063,7 @@ int mgbvh_set_sample_output(mgbvh_ctx* ctx, float* d_samples, uint32_t capacity,
     ctx->learn_count = d_samples ? d_count : nullptr;
     if (ctx->graph_exec) {
         cudaSetDevice(ctx->device);
-        cudaGraphExecDestroy(ctx->graph_exec);
-        ctx->graph_exec = nullptr;
-        ctx->graph_sig.clear();
+        drop_graph(ctx);
     }
     return MGBVH_OK;
 }
@@ -5079,9 +5073,7 @@ int mgbvh_set_graph_capture(mgbvh_ctx* ctx, int enable) {
     ctx->graph_mode = enable != 0;
     if (!ctx->graph_mode && ctx->graph_exec) {
         cudaSetDevice(ctx->device);
-        cudaGraphExecDestroy(ctx->graph_exec);
-        ctx->graph_exec = nullptr;
-        ctx->graph_sig.clear();
+        drop_graph(ctx);
     }
     return MGBVH_OK;
 }
