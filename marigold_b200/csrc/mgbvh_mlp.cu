@@ -339,15 +339,10 @@ int mgbvh_mlp_train_step_dev(const float* d_features, const uint32_t* d_labels, 
                              float* d_loss, void* stream) {
     if (!d_features || !d_labels || !d_gains || !d_weights_bf16 || !d_grad || !d_loss || batch == 0)
         return MGBVH_ERR_INVALID_ARG;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(TrainSmem)) != cudaSuccess ||
-            cudaFuncSetAttribute(forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(TrainSmem)) != cudaSuccess)
-            return MGBVH_ERR_CUDA;
-        attr = true;
-    }
+    // (a limit of the current device and context, so set on every call)
+    if (cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(TrainSmem)) != cudaSuccess)
+        return MGBVH_ERR_CUDA;
     train_kernel<<<(batch + kSB - 1) / kSB, kThreads, sizeof(TrainSmem),
                    reinterpret_cast<cudaStream_t>(stream)>>>(
         d_features, d_labels, d_gains, batch, static_cast<const __nv_bfloat16*>(d_weights_bf16), d_grad,
