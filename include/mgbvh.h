@@ -425,7 +425,9 @@ typedef struct mgbvh_scene_instance {
    triangle array in that BLAS build's permuted order, as vertex index
    triples relative to the mesh's vertex_offset. Lens arrays (NULL = one
    object per leaf) are node-aligned with their node arrays. Gathers the
-   triangles with their vertices. */
+   triangles with their vertices. A TLAS or a mesh's BLAS of more than 2^31
+   nodes, or of more than 2^31 objects without lens, gives
+   MGBVH_ERR_UNSUPPORTED. */
 MGBVH_API int mgbvh_tracer_set_scene_dev(mgbvh_tracer* tracer, const mgbvh_node* d_tlas_nodes,
                                          uint32_t tlas_node_count, const uint32_t* d_tlas_lens,
                                          const mgbvh_scene_instance* d_instances, uint32_t instance_count,

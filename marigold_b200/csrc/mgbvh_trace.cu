@@ -204,6 +204,12 @@ __device__ __forceinline__ void load_node(const float4* __restrict__ nodes, uint
 // leaf by its first triangle (one object per leaf) or its node, 0 for nothing.
 constexpr uint32_t kLeafRef = 0x80000000u;
 
+// Whether references of 31 bits hold the nodes of a tree and, where its leaves
+// have one object each (no lens), the objects.
+bool refs_fit(uint64_t nodes, uint32_t objects, bool has_lens) {
+    return nodes <= kLeafRef && (has_lens || objects <= kLeafRef);
+}
+
 template <bool kLens>
 __device__ __forceinline__ uint32_t node_ref(const float4& lo, const float4& hi, uint32_t node) {
     const uint32_t child = __float_as_uint(hi.w);
@@ -1524,7 +1530,7 @@ int mgbvh_trace_closest_dev(mgbvh_tracer* t, const float* d_rays, uint32_t n_ray
     const float4* rays = reinterpret_cast<const float4*>(d_rays);
     const uint32_t* order = ray_order(t, rays, n_rays, sm, MGBVH_RAY_SORT_BINARY);
     Counts* cnt = out_counts ? t->d_counts : nullptr;
-    if (t->node_count < kLeafRef) {
+    if (refs_fit(t->node_count, t->n_tris, t->lens != nullptr)) {
         cudaMemsetAsync(t->d_next, 0, 4, sm);
         const bool k32 = !(reinterpret_cast<uintptr_t>(nodes) & 31u);  // (nodes are 16-byte aligned)
         int& blocks = t->trace_blocks[4 * (t->lens != nullptr) + 2 * k32 + (cnt != nullptr)];
@@ -1540,7 +1546,7 @@ int mgbvh_trace_closest_dev(mgbvh_tracer* t, const float* d_rays, uint32_t n_ray
             t->lens ? go(trace_persistent_kernel<true, true, false>) : go(trace_persistent_kernel<false, true, false>);
         else
             t->lens ? go(trace_persistent_kernel<true, false, false>) : go(trace_persistent_kernel<false, false, false>);
-    } else if (t->lens) {  // nodes past the references' 31 bits
+    } else if (t->lens) {  // past the references' 31 bits
         trace_kernel<true><<<grid, 128, 0, sm>>>(nodes, t->lens, t->tris, rays, n_rays, d_hit_t, d_hit_prim, cnt,
                                                  t->d_err, order);
     } else {
@@ -1595,6 +1601,11 @@ int mgbvh_tracer_set_scene_dev(mgbvh_tracer* t, const mgbvh_node* d_tlas_nodes, 
         mesh_count == 0 || mesh_count > 65535 || !d_blas_nodes || blas_node_count == 0 || !d_vertices ||
         !d_triangles || triangle_count == 0 || vertex_stride_bytes < 12 || vertex_stride_bytes % 4)
         return MGBVH_ERR_INVALID_ARG;
+    // a tree over n objects has at most 2n - 1 nodes, however long its array
+    auto fits = [](uint32_t nodes, uint32_t objects, bool has_lens) {
+        return refs_fit(std::min<uint64_t>(nodes, 2ull * objects - 1ull), objects, has_lens);
+    };
+    if (!fits(tlas_node_count, instance_count, d_tlas_lens != nullptr)) return MGBVH_ERR_UNSUPPORTED;
     if (cudaSetDevice(t->device) != cudaSuccess) return MGBVH_ERR_CUDA;
     const cudaStream_t sm = reinterpret_cast<cudaStream_t>(stream);
     // the mesh table: checked on the host, copied into the tracer
@@ -1608,6 +1619,8 @@ int mgbvh_tracer_set_scene_dev(mgbvh_tracer* t, const mgbvh_node* d_tlas_nodes, 
         if (m.triangle_count == 0) continue;  // an empty mesh has no BLAS; its instances hit nothing
         if ((uint64_t)m.triangle_offset + m.triangle_count > triangle_count || m.blas_root >= blas_node_count)
             return MGBVH_ERR_INVALID_ARG;
+        if (!fits(blas_node_count - m.blas_root, m.triangle_count, d_blas_lens != nullptr))
+            return MGBVH_ERR_UNSUPPORTED;
         max_count = std::max(max_count, m.triangle_count);
     }
     const size_t need = sizeof(TriRec) * (size_t)triangle_count;
