@@ -531,7 +531,7 @@ __device__ __forceinline__ SweepResult sweep_bins(uint32_t* wb, const BinMap* ma
         const float sa_gt = surface_area(unkey_lo(w[0]), unkey_lo(w[1]), unkey_lo(w[2]), unkey_hi(w[3]),
                                          unkey_hi(w[4]), unkey_hi(w[5]));
         if (map[a].ok && lane >= 1u && lane < map[a].bins && nl >= P.min_leaf && ng >= P.min_leaf) {
-            // (positive, infinite or the default NaN: the bits order as total_cmp)
+            // (never negative: the bits order as the costs do)
             const uint32_t ck = __float_as_uint(area.split_cost(sa_lt[a], sa_gt, nl, ng));
             if (ck < best) {
                 best = ck;
@@ -1000,8 +1000,8 @@ __device__ void warp_build_subtree(const float* lo, const float* hi, uint32_t id
                 if (n >= 8u) cut[a] = p;
             }
         }
-        // costs are positive, infinite or the default NaN: their bits order
-        // as total_cmp does, all below "none"
+        // costs are never negative (ordered_cost): their bits order as they do,
+        // all below "none"
         uint32_t best = kNoKey, win = 0;
 #pragma unroll
         for (uint32_t a = 0; a < 3; ++a) {

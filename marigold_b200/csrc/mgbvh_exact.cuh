@@ -68,11 +68,18 @@ __device__ __forceinline__ float surface_area6(const float* b) {
     return surface_area(b[0], b[1], b[2], b[3], b[4], b[5]);
 }
 
+// A split's cost as the comparisons take it. Costs are 1 or more, infinite, or
+// NaN: infinite over infinite areas, or zero over zero. The reference's NaN
+// has its sign bit set and so comes before every other cost in total_cmp;
+// CUDA's has not and would come after them. It is replaced by 0, which comes
+// first as a float, as its bits and as fkey.
+__device__ __forceinline__ float ordered_cost(float cost) { return cost == cost ? cost : 0.0f; }
+
 __device__ __forceinline__ float split_cost(float sa_lt, float sa_gt, float sa_p, uint32_t n_lt,
                                             uint32_t n_gt) {
     const float lt = __fmul_rn(__fmul_rn(__fdiv_rn(sa_lt, sa_p), kObjectCost), __uint2float_rn(n_lt));
     const float gt = __fmul_rn(__fmul_rn(__fdiv_rn(sa_gt, sa_p), kObjectCost), __uint2float_rn(n_gt));
-    return __fadd_rn(__fadd_rn(kDepthCost, lt), gt);
+    return ordered_cost(__fadd_rn(__fadd_rn(kDepthCost, lt), gt));
 }
 
 // The parent's surface area as a divisor of many areas: the cost above, bit
@@ -111,7 +118,7 @@ struct NodeArea {
         }
         l = __fmul_rn(l, __fmul_rn(kObjectCost, __uint2float_rn(n_lt)));
         g = __fmul_rn(g, __fmul_rn(kObjectCost, __uint2float_rn(n_gt)));
-        return __fadd_rn(__fadd_rn(kDepthCost, l), g);
+        return ordered_cost(__fadd_rn(__fadd_rn(kDepthCost, l), g));
     }
 };
 
