@@ -95,9 +95,13 @@ struct NodeArea {
     float area, rcp;
     bool fast;
 
+    __device__ __forceinline__ static bool in_range(float x) {
+        return x >= 8.673617379884035e-19f && x <= 1.152921504606847e18f;
+    }
+
     __device__ __forceinline__ explicit NodeArea(const float* box) {
         area = surface_area6(box);
-        fast = area >= 8.673617379884035e-19f && area <= 1.152921504606847e18f;
+        fast = in_range(area);
         rcp = __frcp_rn(fast ? area : 1.0f);
     }
 
@@ -108,17 +112,15 @@ struct NodeArea {
     }
 
     __device__ __forceinline__ float split_cost(float sa_lt, float sa_gt, uint32_t n_lt, uint32_t n_gt) const {
-        float l, g;
-        if (fast && fminf(sa_lt, sa_gt) >= 8.673617379884035e-19f && fmaxf(sa_lt, sa_gt) <= 1.152921504606847e18f) {
-            l = ratio(sa_lt);
-            g = ratio(sa_gt);
-        } else {
-            l = __fdiv_rn(sa_lt, area);
-            g = __fdiv_rn(sa_gt, area);
-        }
+        if (fast && in_range(sa_lt) && in_range(sa_gt))  // (no NaN in, none out)
+            return sum(ratio(sa_lt), ratio(sa_gt), n_lt, n_gt);
+        return ordered_cost(sum(__fdiv_rn(sa_lt, area), __fdiv_rn(sa_gt, area), n_lt, n_gt));
+    }
+
+    __device__ __forceinline__ static float sum(float l, float g, uint32_t n_lt, uint32_t n_gt) {
         l = __fmul_rn(l, __fmul_rn(kObjectCost, __uint2float_rn(n_lt)));
         g = __fmul_rn(g, __fmul_rn(kObjectCost, __uint2float_rn(n_gt)));
-        return ordered_cost(__fadd_rn(__fadd_rn(kDepthCost, l), g));
+        return __fadd_rn(__fadd_rn(kDepthCost, l), g);
     }
 };
 

@@ -52,6 +52,21 @@ def test_a_root_of_no_area(oracle, gpu_ctx, n, kind, kw):
                oracle.build(aabbs=boxes, root_bounds=bounds, **kw))
 
 
+@pytest.mark.parametrize("kw", PROFILES)
+@pytest.mark.parametrize("n", SIZES)
+def test_extents_that_overflow(oracle, gpu_ctx, n, kw):
+    """Flat boxes that span more than the largest float: areas are zero times
+    infinite, under a root area that is an ordinary number or none of it."""
+    rng = np.random.default_rng(n)
+    lo = rng.uniform(-3.3e38, 3.3e38, (n, 3))
+    boxes = np.concatenate([lo, np.minimum(lo + rng.uniform(0, 1e37, (n, 3)), 3.3e38)], 1)
+    boxes[:, [1, 4]] = 0
+    boxes = boxes.astype(np.float32) + np.float32(0.0)
+    for bounds in (None, [0.0] * 3 + [1.0] * 3, [0.0] * 6):
+        _check(gpu_build(gpu_ctx, aabbs=boxes, root_bounds=bounds, profiling=False, **kw),
+               oracle.build(aabbs=boxes, root_bounds=bounds, **kw))
+
+
 @pytest.mark.parametrize("queue", [False, True])
 def test_areas_that_overflow_in_a_batch(oracle, queue):
     import torch
