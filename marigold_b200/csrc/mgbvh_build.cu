@@ -8,10 +8,12 @@
 //                               lvl_bin   per-tile 3x32-bin histograms of
 //                                         counts and AABBs in shared memory,
 //                                         merged across tiles with atomics
-//                               lvl_eval  one warp per node: prefix/suffix
-//                                         sweeps, SAH costs, argmin, children
-//                               lvl_part  stable scan partition of the
-//                                         node's 32-byte object records
+//                               lvl_part  decides the node's split (prefix /
+//                                         suffix sweeps, SAH costs, argmin),
+//                                         writes the children, and partitions
+//                                         the 32-byte object records stably
+//                               lvl_eval  the decision as a pass of its own,
+//                                         for the learned form and samples
 //   medium (33..kMediumMax)     one CTA per node builds the whole subtree
 //                               with records in shared memory, warps per
 //                               sub-node, 16-bit index partitions
@@ -54,7 +56,7 @@ constexpr uint32_t kTileMax = 2560;    // most objects of a level-pass tile (til
 constexpr int kMediumWarps = MGBVH_MEDIUM_WARPS;
 constexpr int kMediumThreads = kMediumWarps * 32;
 // Warps of the subtree CTA where there are too few subtrees to fill the SMs
-// with CTAs of kMediumWarps (medium_wide).
+// with CTAs of kMediumWarps (the rule stands at the launch, run_pipeline).
 constexpr int kWideWarps = 8;
 constexpr int kWidestWarps = 16;
 constexpr uint32_t kBinWords = 3 * 32 * 7;  // [axis][bin]{count, lo key xyz, hi key xyz}
@@ -67,7 +69,7 @@ __host__ __device__ __forceinline__ uint32_t lvl_free(uint32_t lv) { return lv =
 
 struct Rec {
     float4 lo;  // min xyz, object id (bits)
-    float4 hi;  // max xyz, 0
+    float4 hi;  // max xyz; w is not read (a subtree CTA keeps bin codes there)
 };
 
 // A record read through L2 only. Within one launch of the persistent batched
@@ -1455,7 +1457,7 @@ __global__ void __launch_bounds__(kTileThreads, MGBVH_PART_MIN_BLOCKS) lvl_part_
 //
 // median_split (bvh/src/lib.rs:444-491) on axes 0, 1 and 2 in turn over the
 // same list (:527-531), for the level-pass nodes whose binned sweeps all
-// refused (lvl_eval_kernel queues them). The waiting nodes' objects form one
+// refused (queue_median). The waiting nodes' objects form one
 // element range, node s owning elements moff[s] .. moff[s+1] in list order.
 // Per axis:
 //   med_key_kernel      (node, centroid key) per element, position as value
@@ -3892,7 +3894,7 @@ int run_pipeline(mgbvh_ctx* ctx, const Caps& C, const Params& P, const Out& O, R
 }
 
 // Forced medians of level-pass nodes (the median kernels above). The nodes
-// that lvl_eval_kernel queued during the pipeline are split here, then their
+// that queue_median listed during the pipeline are split here, then their
 // subtrees are built by another pipeline run, which may queue further nodes;
 // until none is left. The waiting subtrees are disjoint from everything the
 // pipeline built, and their node slots follow from the closed-form numbering,

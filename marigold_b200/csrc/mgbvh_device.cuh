@@ -836,8 +836,7 @@ struct MedianIo {
 // median_split (bvh/src/lib.rs:444-491, 528-530) of the segments whose lanes
 // have `odd`: on axes 0, 1, 2 in turn over the same list, stable; the halves
 // are those of the final (axis-2) order, their boxes the cheapest axis's. All
-// lanes take part. Rare: kept out of line, so that its registers are not the
-// main loop's.
+// lanes take part. Rare: nodes that no threshold or bin tells apart.
 __device__ __forceinline__ void median_segments(bool odd, uint32_t s, uint32_t n, uint32_t m, uint32_t ss, uint32_t se,
                                              uint32_t maxn, SubtreeSmem& T, MedianIo& io) {
     const SubtreeRegs R = io.regs;
@@ -917,7 +916,7 @@ __device__ __forceinline__ void median_segments(bool odd, uint32_t s, uint32_t n
 // instructions on the level-8 icosphere's 59,272 subtrees (22 objects, 5.1
 // depths each): 0.544 ms. With the orders sorted once per subtree (about 1,500
 // instructions) and 36 mask-and-shuffle reads per lane and depth (700-900
-// instructions a depth) it is 329M: 0.386 ms. The general profiles use the same
+// instructions a depth) it is 321M: 0.386 ms. The general profiles use the same
 // tables in place of a depth-first form with one node at a time: 65,536 random
 // triangles at 16 bins, 0.325 -> 0.047 ms; 16.8M mixed triangles, 8.3 -> 5.3 ms.
 template <bool kGeneral>
@@ -1089,7 +1088,7 @@ __device__ void warp_build_subtree(const float* lo, const float* hi, uint32_t id
                 if (lane == s) n_median++;
             }
             if (__any_sync(kFull, odd)) {
-                MedianIo io;  // passed by address: copies, so that the loop's own stay in registers
+                MedianIo io;
                 io.word = word;
                 io.regs = R;
 #pragma unroll
